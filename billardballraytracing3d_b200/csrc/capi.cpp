@@ -55,6 +55,7 @@ cudaError_t sort_requests(const NewtonRequest* req, long long n, const unsigned*
 cudaError_t ray_order(const double* o, const double* d, long long n, const double center[3], double radius,
                       void* ws, int* order, cudaStream_t stream, bool entry, long long base);
 cudaError_t launch_query(const DScene& S, const QueryArgs& Q, cudaStream_t stream);
+cudaError_t launch_leaf_records(const DScene& S, int n_slots, float4* out, cudaStream_t st);
 cudaError_t noalloc_prepare();
 cudaError_t launch_trace_noalloc(const DScene& S, TraceArgs A, bool count_hits, long long* hit_counts_out,
                                  long long* host_stats, cudaStream_t stream, int sm_count);
@@ -420,6 +421,19 @@ int upload_node_tables(bbrt_scene* s, const std::vector<double>& nbox, const std
     return BBRT_OK;
 }
 
+// The leaf records (DScene::leaf_rec) of a scene or set whose leaf order,
+// object tables and cull boxes are on the device; ready when this returns.
+int build_leaf_records(bbrt_scene* s) {
+    const size_t n = s->host.leaf_objects.size();
+    float4* rec = nullptr;
+    int rc = s->alloc(2 * n, rec);
+    if (rc) return rc;
+    BBRT_CUDA(bbrt::launch_leaf_records(s->dev, static_cast<int>(n), rec, s->stream));
+    BBRT_CUDA(cudaStreamSynchronize(s->stream));
+    s->dev.leaf_rec = rec;
+    return BBRT_OK;
+}
+
 int ensure_uploaded(bbrt_scene* s) {
     if (s->uploaded) return BBRT_OK;
     int rc0 = ensure_device(s);
@@ -522,6 +536,7 @@ int ensure_uploaded(bbrt_scene* s) {
     for (const void* p : std::initializer_list<const void*>{ D.node_box, D.c_cell, D.c_cell_box, D.c_block_box })
         if (reinterpret_cast<uintptr_t>(p) % 16 != 0)
             return fail(BBRT_ERR_CUDA, "bbrt_scene_upload: scene array not 16-byte aligned");
+    if ((rc = build_leaf_records(s))) return rc;
     BBRT_CUDA(s->stats.ensure(sizeof(long long) * bbrt::ST_COUNT));
     BBRT_CUDA(s->work.ensure(sizeof(unsigned long long)));
     s->uploaded = true;
@@ -2842,6 +2857,7 @@ int build_scene_set(const std::vector<bbrt_scene*>& mem, bbrt_scene_set* set) {
         if ((rc = join_device(S, bb, D.c_block_box))) return rc;
     }
     BBRT_CUDA(cudaStreamSynchronize(S.stream));
+    if ((rc = build_leaf_records(&S))) return rc;
     BBRT_CUDA(S.stats.ensure(sizeof(long long) * bbrt::ST_COUNT));
     BBRT_CUDA(S.work.ensure(sizeof(unsigned long long)));
     S.tables_uploaded = true;

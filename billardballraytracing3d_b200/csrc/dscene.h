@@ -30,6 +30,12 @@ struct DScene {
     const int* node_link = nullptr;        // [n_nodes][4]  internal: left, right, 0, axis
                                            //               leaf:     start, -1, count, 0
     const int* leaf_objects = nullptr;
+    // Leaf records, one per leaf slot (leaf_objects order), 32 bytes each as
+    // two 16-byte halves: the object's stage-1 cull box (min xyz, max xyz:
+    // the union of the patch's block boxes; -inf / +inf for a triangle or
+    // without cull tables), then its patch index (or ~triangle index) and its
+    // object index, both as int bits.
+    const float4* leaf_rec = nullptr;
     int smem_nodes = 0;                    // nodes [0, smem_nodes) staged in shared memory
     // FP32 copies of the node boxes (nearest rounding) for the FP32 node
     // test, and per axis a bound on |coordinate| over every node box (FP32,

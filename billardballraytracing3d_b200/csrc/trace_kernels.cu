@@ -113,6 +113,40 @@ __device__ __forceinline__ bool cull_box(const float* __restrict__ b, const Cull
     return tmin <= tmax;
 }
 
+// One leaf slot's record (DScene::leaf_rec).
+struct LeafRec {
+    float4 a, b;   // min xyz, max x | max yz, sub, object
+    __device__ __forceinline__ int sub() const { return __float_as_int(b.z); }
+    __device__ __forceinline__ int obj() const { return __float_as_int(b.w); }
+};
+
+__device__ __forceinline__ LeafRec load_leaf(const DScene& S, int slot) {
+    LeafRec r;
+    r.a = S.leaf_rec[2LL * slot];
+    r.b = S.leaf_rec[2LL * slot + 1];
+    return r;
+}
+
+// cull_box against a leaf record's box: a patch whose box fails has no block,
+// cell or triangle that passes (the box is their union), so stage 1 misses.
+// About two thirds of the patches of a visited leaf end here, for one box
+// test and two 16-byte loads instead of 16 block boxes.
+__device__ __forceinline__ bool cull_leaf(const LeafRec& r, const CullRay& c) {
+    float t1 = (r.a.x - c.delta - c.ox) * c.ix, t2 = (r.a.w + c.delta - c.ox) * c.ix;
+    float tmin = fmaxf(0.0f, fminf(t1, t2)), tmax = fmaxf(t1, t2);
+    t1 = (r.a.y - c.delta - c.oy) * c.iy; t2 = (r.b.x + c.delta - c.oy) * c.iy;
+    tmin = fmaxf(tmin, fminf(t1, t2)); tmax = fminf(tmax, fmaxf(t1, t2));
+    t1 = (r.a.z - c.delta - c.oz) * c.iz; t2 = (r.b.y + c.delta - c.oz) * c.iz;
+    tmin = fmaxf(tmin, fminf(t1, t2)); tmax = fminf(tmax, fmaxf(t1, t2));
+    return tmin <= tmax;
+}
+
+// The n-th (from 0) set bit of m, which has more than n.
+__device__ __forceinline__ int nth_bit(unsigned m, int n) {
+    for (int k = 0; k < n; ++k) m &= m - 1u;
+    return __ffs(m) - 1;
+}
+
 // FP32 BVH node test that reproduces ray_box_exact's decision or defers it.
 //
 // ray_box_exact(o, 1/d, box, best_t) passes exactly when, over the three
@@ -330,7 +364,13 @@ __device__ QHit bvh_query(const DScene& S, const V3& o, const V3& d, int cull_fl
         if (link[1] < 0) {
             const int start = link[0], count = link[2];
             for (int k = 0; k < count; ++k) {
-                const int obj = S.leaf_objects[start + k];
+                const LeafRec rec = load_leaf(S, start + k);
+                const int obj = rec.obj();
+                if (use_cull && rec.sub() >= 0 && !cull_leaf(rec, cr)) {
+                    ++ctr.patch_tests;
+                    ++ctr.cell_tests;
+                    continue;
+                }
                 QHit h;
                 const int r = object_intersect(S, obj, o, d, use_cull, cr, h, ctr);
                 if (off_patch_miss && h.err == BBRT_RAY_NEWTON_DOMAIN) {
@@ -648,8 +688,7 @@ __device__ __forceinline__ void warp_cell_tris(const double* X, const double* CC
     for (int p0 = 0; p0 < total; p0 += 32) {
         const int p = p0 + lane;
         if (p < total) {
-            const int bit = __fns(cm, 0, p / 6 + 1);
-            const int c = c0 + bit;
+            const int c = c0 + nth_bit(cm, p / 6);
             stage1_tri(X, CC, n, base_i + c / w, base_j + c % w, p % 6, o, d, best);
         }
     }
@@ -749,7 +788,7 @@ __device__ Stage1 group_patch_stage1(const DScene& S, int pidx, const V3& o, con
                     for (int p0 = 0; p0 < total; p0 += WH) {
                         const int p = p0 + hl;
                         if (p < total) {
-                            const int cell = c0 + __fns(cm, 0, p / 6 + 1);
+                            const int cell = c0 + nth_bit(cm, p / 6);
                             stage1_tri(X, CC, n, i0 + cell / w, j0 + cell % w, p % 6, o, d, best);
                         }
                     }
@@ -1030,13 +1069,23 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
                 }
             }
         } else if (mode == M_LEAF) {
+            // patches whose box the ray misses end here (not while samples are
+            // recorded: their stage-1 misses are training samples)
+            LeafRec rec;
+            while (q.leaf_k < q.leaf_count) {
+                rec = load_leaf(S, q.leaf_start + q.leaf_k);
+                if (rec.sub() < 0 || !q.use_cull || A.samples || cull_leaf(rec, q.cr)) break;
+                ++cray.patch_tests;
+                ++cray.cell_tests;
+                ++q.leaf_k;
+            }
             if (q.leaf_k >= q.leaf_count) {
                 mode = M_NODE;
             } else {
-                const int obj = S.leaf_objects[q.leaf_start + q.leaf_k];
-                if (S.obj_kind[obj] != BBRT_OBJ_PATCH) {
+                const int obj = rec.obj();
+                if (rec.sub() < 0) {
                     QHit h;
-                    if (triangle_intersect(S, S.obj_sub[obj], r.o, r.d, h, cray) && h.t < q.best_t) {
+                    if (triangle_intersect(S, ~rec.sub(), r.o, r.d, h, cray) && h.t < q.best_t) {
                         q.best_t = h.t;
                         if (q.best_ver < static_cast<int>(kStackAlways)) ++q.best_ver;
                         q.best_obj = obj;
@@ -1072,11 +1121,11 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
                         // (instances with G > 1 run only with the warp-cooperative
                         // stage 1, so they carry no per-lane stage-1 modes)
                         q.obj = obj;
-                        q.pidx = S.obj_sub[obj];
+                        q.pidx = rec.sub();
                         mode = M_S1_WARP;
                     } else {
                         q.obj = obj;
-                        q.pidx = S.obj_sub[obj];
+                        q.pidx = rec.sub();
                         q.s1.have = false;
                         ++cray.patch_tests;
                         if (q.use_cull) {
@@ -1211,8 +1260,9 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
 #pragma unroll
                 for (int g = 0; g < G; ++g) pend &= pend - 1;
                 const int gg = lane / WH;
-                const unsigned pos = __fns(batch, 0, gg + 1);
-                const int src = pos < 32u ? static_cast<int>(pos) : __ffs(batch) - 1;
+                unsigned mine = batch;
+                for (int g = 0; g < gg; ++g) mine &= mine - 1;
+                const int src = __ffs(mine ? mine : batch) - 1;
                 V3 so, sd;
                 so.x = __shfl_sync(kFull, r.o.x, src);
                 so.y = __shfl_sync(kFull, r.o.y, src);
@@ -1246,8 +1296,10 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
                         ct = __shfl_sync(kFull, c2.cell_tests, leader);
                         tt = __shfl_sync(kFull, c2.tri_tests, leader);
                     }
-                    const unsigned owner = __fns(batch, 0, hv + 1);
-                    if (owner < 32u && lane == static_cast<int>(owner)) {
+                    unsigned left = batch;
+#pragma unroll
+                    for (int g = 0; g < hv; ++g) left &= left - 1;
+                    if (left && lane == __ffs(left) - 1) {
                         q.s1.have = have != 0;
                         q.s1.t = st;
                         q.s1.key = sk;
@@ -1599,14 +1651,32 @@ __device__ QHit warp_bvh_query(const DScene& S, const V3& o, const V3& d, int cu
         const int* link = in_smem ? slink + 4 * idx : S.node_link + 4LL * idx;
         if (link[1] < 0) {
             const int start = link[0], count = link[2];
-            for (int k = 0; k < count; ++k) {
-                const int obj = S.leaf_objects[start + k];
+            // lane k takes slot k's box; only the objects that pass are tried, in order
+            for (int k0 = 0; k0 < count; k0 += 32) {
+              LeafRec rec;
+              bool try_it = false, culled = false;
+              if (k0 + lane < count) {
+                  rec = load_leaf(S, start + k0 + lane);
+                  try_it = rec.sub() < 0 || !use_cull || cull_leaf(rec, cr);
+                  culled = !try_it;
+              }
+              if constexpr (Ctr::kOn) {
+                  const int nc = __popc(__ballot_sync(kFull, culled));
+                  if (lane == 0) {
+                      ctr.patch_tests += nc;
+                      ctr.cell_tests += nc;
+                  }
+              }
+              for (unsigned todo = __ballot_sync(kFull, try_it); todo; todo &= todo - 1) {
+                const int src = __ffs(todo) - 1;
+                const int obj = __shfl_sync(kFull, rec.obj(), src);
+                const int sub = __shfl_sync(kFull, rec.sub(), src);
                 QHit h;
                 h.err = 0;
                 h.ev0 = h.ev1 = 0.0;
                 int r = 0;
-                if (S.obj_kind[obj] == BBRT_OBJ_PATCH) {
-                    const int pidx = S.obj_sub[obj];
+                if (sub >= 0) {
+                    const int pidx = sub;
                     const Stage1 s1 = warp_patch_stage1(S, pidx, o, d, use_cull, cr, lane, ctr);
                     if (s1.have) {
                         double u0, v0;
@@ -1622,7 +1692,7 @@ __device__ QHit warp_bvh_query(const DScene& S, const V3& o, const V3& d, int cu
                     }
                 } else {
                     CountersT<false> dummy;
-                    r = triangle_intersect(S, S.obj_sub[obj], o, d, h, dummy);
+                    r = triangle_intersect(S, ~sub, o, d, h, dummy);
                 }
                 if (off_patch_miss && h.err == BBRT_RAY_NEWTON_DOMAIN) {
                     if (lane == 0) ++ctr.off_patch;
@@ -1637,6 +1707,7 @@ __device__ QHit warp_bvh_query(const DScene& S, const V3& o, const V3& d, int cu
                     best = h;
                     best.obj = obj;
                 }
+              }
             }
             continue;
         }
@@ -2072,6 +2143,34 @@ cudaError_t launch_resume_warp(const DScene& S, const TraceArgs& A, const WaveAr
         case 3: return launch_resume_warp_shape<2>(S, A, W, reqs, rays, n, sm_count, 1536, stream);
         default: return launch_resume_warp_shape<3>(S, A, W, reqs, rays, n, sm_count, 0, stream);
     }
+}
+
+// Leaf records (DScene::leaf_rec) from the leaf order and the cull tables: one
+// thread per leaf slot.
+__global__ void k_leaf_records(DScene S, int n_slots, float4* __restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n_slots) return;
+    const int obj = S.leaf_objects[k], sub = S.obj_sub[obj];
+    const bool patch = S.obj_kind[obj] == BBRT_OBJ_PATCH;
+    float lo[3] = { -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F }, hi[3] = { CUDART_INF_F, CUDART_INF_F, CUDART_INF_F };
+    const int nb = S.n_blocks_side * S.n_blocks_side;
+    if (patch && S.c_block_box && nb > 0) {
+        const float* b = S.c_block_box + 6LL * nb * sub;
+        for (int a = 0; a < 3; ++a) { lo[a] = b[a]; hi[a] = b[3 + a]; }
+        for (int j = 1; j < nb; ++j)
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = fminf(lo[a], b[6 * j + a]);
+                hi[a] = fmaxf(hi[a], b[6 * j + 3 + a]);
+            }
+    }
+    out[2LL * k] = make_float4(lo[0], lo[1], lo[2], hi[0]);
+    out[2LL * k + 1] = make_float4(hi[1], hi[2], __int_as_float(patch ? sub : ~sub), __int_as_float(obj));
+}
+
+cudaError_t launch_leaf_records(const DScene& S, int n_slots, float4* out, cudaStream_t st) {
+    if (n_slots <= 0) return cudaSuccess;
+    k_leaf_records<<<static_cast<unsigned>((n_slots + 127) / 128), 128, 0, st>>>(S, n_slots, out);
+    return cudaGetLastError();
 }
 
 // ---- BounceMapDriver::run on the device ------------------------------------
