@@ -671,7 +671,7 @@ struct Tuning {
     int log_rounds = 0;               // print per-round counts and times to stderr
     int warp_tail = 1;                // finish the tail one warp per ray (else one thread per ray)
     int advance_shape = 3;            // k_advance launch shape (see launch_advance): 512 threads x 1 block per SM
-    int warp_stage1 = 1;              // k_advance runs each patch's stage 1 with the whole warp
+    int warp_stage1 = 1;              // reported only: k_advance always runs stage 1 by the warp
     int resume_queries = 1;           // suspended queries resume where they stopped (else replay from the root)
     int tail_shape = 0;               // k_resume_warp launch shape (see launch_resume_warp)
     int group_newton = 0;             // k_newton by 8-lane groups (exact, measured slower: off)
@@ -679,9 +679,6 @@ struct Tuning {
     int sort_requests = 1;            // group each round's Newton requests by patch before solving them
     int sort_side = 4;                // ... and within a patch by the side x side region of the stage-1 cell
     int order_entry = 1;              // round-0 order keyed on the scene-sphere entry point (else the origin)
-    int child_test = -1;              // k_advance child tests: -1 when the BVH exceeds the staged nodes, 0 / 1
-    int half_stage1 = 1;              // k_advance stage 1 of two patches at a time by half-warps
-    int quarter_stage1 = 0;           // ... four at a time by quarter-warps
     int node_f32 = 1;                 // BVH nodes tested in FP32, FP64 where FP32 cannot decide (k_advance, tail)
     int adapt_lanes = 1;              // small k_advance rounds: fewer rays per warp, over every warp
     long long newton_group_max = 32768;  // smaller Newton rounds: 8 lanes per request
@@ -707,9 +704,6 @@ const Tuning& tuning() {
         if (const char* e = std::getenv("BBRT_SORT_REQ")) v.sort_requests = std::atoi(e);
         if (const char* e = std::getenv("BBRT_SORT_SIDE")) v.sort_side = std::max(1, std::atoi(e));
         if (const char* e = std::getenv("BBRT_ORDER_ENTRY")) v.order_entry = std::atoi(e);
-        if (const char* e = std::getenv("BBRT_CHILD_TEST")) v.child_test = std::atoi(e);
-        if (const char* e = std::getenv("BBRT_HALF_S1")) v.half_stage1 = std::atoi(e);
-        if (const char* e = std::getenv("BBRT_QUARTER_S1")) v.quarter_stage1 = std::atoi(e);
         if (const char* e = std::getenv("BBRT_NODE_F32")) v.node_f32 = std::atoi(e);
         if (const char* e = std::getenv("BBRT_ADAPT_LANES")) v.adapt_lanes = std::atoi(e);
         if (const char* e = std::getenv("BBRT_NEWTON_GROUP_MAX")) v.newton_group_max = std::atoll(e);
@@ -850,11 +844,7 @@ int build_wave_graph(bbrt_scene* s, const bbrt::TraceArgs& A, const bbrt_tuning&
     bbrt::wave_layout(s->wave.p, n, W, req_a, req_b);
     unsigned int* c = static_cast<unsigned int*>(s->wave_ctr.p);
     W.counters = c;
-    W.warp_stage1 = T.warp_stage1;
     W.resume_queries = tuning().resume_queries;
-    W.child_test = tuning().child_test;
-    W.half_stage1 = tuning().half_stage1;
-    W.quarter_stage1 = tuning().quarter_stage1;
     W.node_f32 = tuning().node_f32;
     W.adapt_lanes = tuning().adapt_lanes;
     W.newton_group_max = tuning().newton_group_max;
@@ -984,7 +974,7 @@ int launch_wave_graph(bbrt_scene* s, const bbrt::TraceArgs& A, const bbrt_tuning
                          static_cast<long long>(T.advance_shape), static_cast<long long>(T.warp_stage1),
                          static_cast<long long>(T.order_rays), static_cast<long long>(T.warp_tail), T.wave_tail,
                          static_cast<long long>(tuning().resume_queries), static_cast<long long>(tuning().group_newton),
-                         static_cast<long long>(tuning().tail_shape), static_cast<long long>(tuning().quarter_stage1),
+                         static_cast<long long>(tuning().tail_shape),
                          static_cast<long long>(tuning().node_f32), static_cast<long long>(tuning().adapt_lanes),
                          tuning().newton_group_max, max_rounds,
                          static_cast<long long>(sort_round_requests(s)), watchdog_cycles(T), mma_wait_cycles(T),
@@ -1053,11 +1043,7 @@ struct WaveRun {
         bbrt::wave_layout(s->wave.p, n, W, req_a, req_b);
         if (sort_round_requests(s)) BBRT_CUDA(s->order_ws.ensure(bbrt::ray_order_workspace_bytes(n)));
         W.counters = static_cast<unsigned int*>(s->wave_ctr.p);
-        W.warp_stage1 = T.warp_stage1;
         W.resume_queries = tuning().resume_queries;
-        W.child_test = tuning().child_test;
-        W.half_stage1 = tuning().half_stage1;
-        W.quarter_stage1 = tuning().quarter_stage1;
         W.node_f32 = tuning().node_f32;
         W.adapt_lanes = tuning().adapt_lanes;
         W.newton_group_max = tuning().newton_group_max;

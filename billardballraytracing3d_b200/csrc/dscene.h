@@ -171,7 +171,6 @@ constexpr int kResData = 11;
 struct WaveArgs {
     double* o = nullptr;       // [n][3] ray state between rounds
     double* d = nullptr;
-    double* end = nullptr;
     int* bounces = nullptr;
     int* nres = nullptr;
     int* res_obj = nullptr;    // [n][kResolved]
@@ -189,21 +188,16 @@ struct WaveArgs {
     const double* frame = nullptr;             // per-patch frames (size L at [12] of each 16)
     double guess_min_logit = 0.0;              // confidence needed to start Newton from the guess
     double guess_t_window = 0.5;               // accepted |t - t_stage1| in units of L
-    int warp_stage1 = 1;                       // stage 1 of k_advance by the whole warp (else per lane)
-    int half_stage1 = 1;                       // ... two patches at a time by half-warps where they fit
-    int quarter_stage1 = 0;                    // ... four at a time by quarter-warps instead
     // Traversal state of a query suspended for a Newton solve, so that the
     // next round resumes it instead of replaying it from the root:
-    // qs_int[ray][kQsInt] = stack depth (-1: none saved), leaf start, leaf
-    // count, position in the leaf, best object, best resolved entry;
-    // qs_dbl[ray][3] = best t, triangle u, v; qs_stack[ray][kSaveStack].
+    // qs_int[ray][kQsInt] = stack depth (-1: none saved), leaf slot, end of the
+    // leaf's slots, best object, best resolved entry; qs_t[ray] = best t;
+    // qs_stack[ray][kSaveStack].
     int* qs_int = nullptr;
-    double* qs_dbl = nullptr;
+    double* qs_t = nullptr;
     int* qs_stack = nullptr;
     int resume_queries = 1;
     int group_newton = 0;                      // Newton solves by 8-lane groups when the patches allow it
-    int child_test = -1;                       // k_advance tests a node's children with it (-1: when the
-                                               // tree is larger than the shared-memory copy)
     // Graph-launched trace: the launch's item count (runnable rays, requests,
     // tail rays) is read from this device word instead of the host argument,
     // and the Newton kernel copies each request it solves to next_req (the
@@ -236,7 +230,7 @@ constexpr int kWcTailNext = 8; // next slot of the tail kernel (rays handed out 
 constexpr int kWcOvfNext = 9;  // next slot of the overflow tail
 constexpr int kWaveCounters = 10;
 
-constexpr int kQsInt = 6;
+constexpr int kQsInt = 5;
 constexpr int kSaveStack = 24;
 
 struct QueryArgs {

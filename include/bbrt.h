@@ -427,7 +427,7 @@ BBRT_API int bbrt_trace_batch(const bbrt_scene_t* scenes, int n_scenes, const do
 typedef struct bbrt_tuning {
     int advance_shape;        /* k_advance launch shape, threads x blocks per SM: 0 = 128x3, 1 = 256x2,
                                  2 = 128x4, 3 = 512x1 (default), 4 = 768x1, 5 = 1024x1, 6 = 384x1 */
-    int warp_stage1;          /* 1 (default): each patch's stage 1 by the whole warp */
+    int warp_stage1;          /* no effect: a patch's stage 1 always runs by the whole warp */
     int order_rays;           /* 1 (default): bucket rays by direction and origin before round 0 */
     int warp_tail;            /* 1 (default): the tail one warp per ray, else one thread per ray */
     long long wave_tail;      /* rays still waiting when the tail takes over (4096) */
