@@ -35,7 +35,8 @@
 #include "scene_host.hpp"
 
 namespace bbrt {
-cudaError_t launch_trace(const DScene& S, const TraceArgs& A, cudaStream_t stream, int sm_count);
+cudaError_t launch_rays(const DScene& S, const TraceArgs& A, const WaveArgs& W, const NewtonRequest* reqs, const int* rays,
+                        long long n, int sm_count, cudaStream_t stream);
 size_t wave_workspace_bytes(long long n);
 void wave_layout(void* ws, long long n, WaveArgs& W, NewtonRequest*& req_a, NewtonRequest*& req_b);
 cudaError_t launch_advance(const DScene& S, const TraceArgs& A, const WaveArgs& W, int sm_count, int shape,
@@ -44,8 +45,6 @@ cudaError_t launch_newton(const DScene& S, const TraceArgs& A, const WaveArgs& W
                           cudaStream_t stream);
 cudaError_t launch_wave_decide(unsigned int* counters, long long wave_tail, long long max_rounds,
                                cudaGraphConditionalHandle loop, cudaStream_t stream);
-cudaError_t launch_resume_warp(const DScene& S, const TraceArgs& A, const WaveArgs& W, const NewtonRequest* reqs,
-                               const int* rays, long long n, int sm_count, int shape, cudaStream_t stream);
 cudaError_t launch_resume(const DScene& S, const TraceArgs& A, const WaveArgs& W, const NewtonRequest* reqs,
                           const int* rays, long long n, cudaStream_t stream);
 size_t ray_order_workspace_bytes(long long n);
@@ -55,6 +54,7 @@ cudaError_t sort_requests(const NewtonRequest* req, long long n, const unsigned*
 cudaError_t ray_order(const double* o, const double* d, long long n, const double center[3], double radius,
                       void* ws, int* order, cudaStream_t stream, bool entry, long long base);
 cudaError_t launch_query(const DScene& S, const QueryArgs& Q, cudaStream_t stream);
+cudaError_t launch_query_warp(const DScene& S, const QueryArgs& Q, int sm_count, cudaStream_t stream);
 cudaError_t launch_leaf_records(const DScene& S, int n_slots, float4* out, cudaStream_t st);
 cudaError_t noalloc_prepare();
 cudaError_t launch_trace_noalloc(const DScene& S, TraceArgs A, bool count_hits, long long* hit_counts_out,
@@ -421,16 +421,102 @@ int upload_node_tables(bbrt_scene* s, const std::vector<double>& nbox, const std
     return BBRT_OK;
 }
 
-// The leaf records (DScene::leaf_rec) of a scene or set whose leaf order,
-// object tables and cull boxes are on the device; ready when this returns.
-int build_leaf_records(bbrt_scene* s) {
-    const size_t n = s->host.leaf_objects.size();
-    float4* rec = nullptr;
-    int rc = s->alloc(2 * n, rec);
+// The leaf tables of DScene (leaf records, and the leaf lists of ray_warp.cu)
+// of a scene or set whose object tables, leaf order and cull boxes are on the
+// device, from its breadth-first node arrays and the root of each tree; one
+// allocation, ready when this returns.
+int build_leaf_tables(bbrt_scene* s, const std::vector<double>& nbox, const std::vector<int>& nlink,
+                      const std::vector<int>& roots) {
+    bbrt::DScene& D = s->dev;
+    constexpr int kCutLeaves = 32, kMaxDepth = 60;
+    const size_t n_slots = s->host.leaf_objects.size(), nn = nlink.size() / 4;
+    std::vector<int> leaf_of(nn, -1), below(nn, 0), leaves, cuts, m_cut{ 0 }, cut_first;
+    bool shallow = true;
+    for (size_t k = nn; k-- > 0;)   // children come after their parent
+        below[k] = nlink[4 * k + 1] < 0 ? 1 : below[nlink[4 * k]] + below[nlink[4 * k + 1]];
+    struct Item { int node, depth; bool cut; };
+    std::vector<Item> stack;
+    for (int root : roots) {
+        if (nn == 0) break;
+        stack.push_back({ root, 0, false });
+        while (!stack.empty()) {
+            Item it = stack.back();
+            stack.pop_back();
+            if (it.depth > kMaxDepth) shallow = false;
+            if (!it.cut && below[it.node] <= kCutLeaves) {
+                cuts.push_back(it.node);
+                cut_first.push_back(static_cast<int>(leaves.size()));
+                it.cut = true;
+            }
+            if (nlink[4 * it.node + 1] < 0) {
+                leaf_of[it.node] = static_cast<int>(leaves.size());
+                leaves.push_back(it.node);
+            } else {
+                stack.push_back({ nlink[4 * it.node + 1], it.depth + 1, it.cut });
+                stack.push_back({ nlink[4 * it.node], it.depth + 1, it.cut });
+            }
+        }
+        m_cut.push_back(static_cast<int>(cuts.size()));
+    }
+    const size_t nl = leaves.size(), ncut = cuts.size();
+    std::vector<int> rank(8 * nl);
+    std::vector<int> walk;
+    for (int oct = 0; oct < 8; ++oct) {
+        int at = 0;
+        for (int root : roots) {
+            if (nn == 0) break;
+            walk.push_back(root);
+            while (!walk.empty()) {
+                const int k = walk.back();
+                walk.pop_back();
+                const int* l = &nlink[4 * static_cast<size_t>(k)];
+                if (l[1] < 0) {
+                    rank[8 * static_cast<size_t>(leaf_of[k]) + oct] = at++;
+                } else {   // the reference's pushes (BVH.hpp:117-125)
+                    const bool neg = oct >> l[3] & 1;
+                    walk.push_back(neg ? l[0] : l[1]);
+                    walk.push_back(neg ? l[1] : l[0]);
+                }
+            }
+        }
+    }
+    auto pad = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
+    const size_t at_rec = 0, at_node = at_rec + pad(32 * n_slots), at_box = at_node + pad(32 * nl),
+                 at_rank = at_box + pad(48 * nl), at_cut = at_rank + pad(32 * nl), at_cbox = at_cut + pad(32 * ncut),
+                 at_m = at_cbox + pad(48 * ncut), total = at_m + pad(sizeof(int) * m_cut.size());
+    std::vector<char> blob(total, 0);
+    auto record = [&](size_t at, int node, int a, int b) {   // FP32 box and two ints
+        float f[6];
+        for (int k = 0; k < 6; ++k) f[k] = static_cast<float>(nbox[6 * static_cast<size_t>(node) + k]);
+        std::memcpy(&blob[at], f, sizeof f);
+        std::memcpy(&blob[at + 24], &a, 4);
+        std::memcpy(&blob[at + 28], &b, 4);
+    };
+    for (size_t l = 0; l < nl; ++l) {
+        const int k = leaves[l];
+        record(at_node + 32 * l, k, nlink[4 * static_cast<size_t>(k)], nlink[4 * static_cast<size_t>(k) + 2]);
+        std::memcpy(&blob[at_box + 48 * l], &nbox[6 * static_cast<size_t>(k)], 48);
+    }
+    for (size_t c = 0; c < ncut; ++c) {
+        record(at_cut + 32 * c, cuts[c], cut_first[c], below[cuts[c]]);
+        std::memcpy(&blob[at_cbox + 48 * c], &nbox[6 * static_cast<size_t>(cuts[c])], 48);
+    }
+    if (nl) std::memcpy(&blob[at_rank], rank.data(), 32 * nl);
+    std::memcpy(&blob[at_m], m_cut.data(), sizeof(int) * m_cut.size());
+    char* d = nullptr;
+    int rc = s->alloc(total, d);
     if (rc) return rc;
-    BBRT_CUDA(bbrt::launch_leaf_records(s->dev, static_cast<int>(n), rec, s->stream));
+    BBRT_CUDA(cudaMemcpyAsync(d, blob.data(), total, cudaMemcpyHostToDevice, s->stream));
+    BBRT_CUDA(bbrt::launch_leaf_records(D, static_cast<int>(n_slots), reinterpret_cast<float4*>(d + at_rec), s->stream));
     BBRT_CUDA(cudaStreamSynchronize(s->stream));
-    s->dev.leaf_rec = rec;
+    D.leaf_rec = reinterpret_cast<const float4*>(d + at_rec);
+    D.leaf_node = reinterpret_cast<const float4*>(d + at_node);
+    D.leaf_box = reinterpret_cast<const double*>(d + at_box);
+    D.leaf_rank = reinterpret_cast<const int*>(d + at_rank);
+    D.cut_rec = reinterpret_cast<const float4*>(d + at_cut);
+    D.cut_box = reinterpret_cast<const double*>(d + at_cbox);
+    D.m_cut = reinterpret_cast<const int*>(d + at_m);
+    D.leaf_lists = D.node_f32_ok && shallow ? 1 : 0;
     return BBRT_OK;
 }
 
@@ -536,7 +622,7 @@ int ensure_uploaded(bbrt_scene* s) {
     for (const void* p : std::initializer_list<const void*>{ D.node_box, D.c_cell, D.c_cell_box, D.c_block_box })
         if (reinterpret_cast<uintptr_t>(p) % 16 != 0)
             return fail(BBRT_ERR_CUDA, "bbrt_scene_upload: scene array not 16-byte aligned");
-    if ((rc = build_leaf_records(s))) return rc;
+    if ((rc = build_leaf_tables(s, nbox, nlink, { 0 }))) return rc;
     BBRT_CUDA(s->stats.ensure(sizeof(long long) * bbrt::ST_COUNT));
     BBRT_CUDA(s->work.ensure(sizeof(unsigned long long)));
     s->uploaded = true;
@@ -673,7 +759,6 @@ struct Tuning {
     int advance_shape = 3;            // k_advance launch shape (see launch_advance): 512 threads x 1 block per SM
     int warp_stage1 = 1;              // reported only: k_advance always runs stage 1 by the warp
     int resume_queries = 1;           // suspended queries resume where they stopped (else replay from the root)
-    int tail_shape = 0;               // k_resume_warp launch shape (see launch_resume_warp)
     int group_newton = 0;             // k_newton by 8-lane groups (exact, measured slower: off)
     int graph_rounds = 1;             // the rounds as one CUDA graph with a device-side loop
     int sort_requests = 1;            // group each round's Newton requests by patch before solving them
@@ -698,7 +783,6 @@ const Tuning& tuning() {
         if (const char* e = std::getenv("BBRT_ADV_SHAPE")) v.advance_shape = std::atoi(e);
         if (const char* e = std::getenv("BBRT_WARP_S1")) v.warp_stage1 = std::atoi(e);
         if (const char* e = std::getenv("BBRT_RESUME")) v.resume_queries = std::atoi(e);
-        if (const char* e = std::getenv("BBRT_TAIL_SHAPE")) v.tail_shape = std::atoi(e);
         if (const char* e = std::getenv("BBRT_GROUP_NEWTON")) v.group_newton = std::atoi(e);
         if (const char* e = std::getenv("BBRT_GRAPH")) v.graph_rounds = std::atoi(e);
         if (const char* e = std::getenv("BBRT_SORT_REQ")) v.sort_requests = std::atoi(e);
@@ -757,7 +841,7 @@ long long mma_wait_cycles(const bbrt_tuning& T) { return T.mma_wait_cycles > 0 ?
 cudaError_t run_tail(bbrt_scene* s, const bbrt::TraceArgs& A, const bbrt::WaveArgs& W,
                      const bbrt::NewtonRequest* reqs, const int* rays, long long n, cudaStream_t st) {
     if (scene_tuning(s).warp_tail)
-        return bbrt::launch_resume_warp(s->dev, A, W, reqs, rays, n, s->sm_count, tuning().tail_shape, st);
+        return bbrt::launch_rays(s->dev, A, W, reqs, rays, n, s->sm_count, st);
     return bbrt::launch_resume(s->dev, A, W, reqs, rays, n, st);
 }
 
@@ -974,7 +1058,6 @@ int launch_wave_graph(bbrt_scene* s, const bbrt::TraceArgs& A, const bbrt_tuning
                          static_cast<long long>(T.advance_shape), static_cast<long long>(T.warp_stage1),
                          static_cast<long long>(T.order_rays), static_cast<long long>(T.warp_tail), T.wave_tail,
                          static_cast<long long>(tuning().resume_queries), static_cast<long long>(tuning().group_newton),
-                         static_cast<long long>(tuning().tail_shape),
                          static_cast<long long>(tuning().node_f32), static_cast<long long>(tuning().adapt_lanes),
                          tuning().newton_group_max, max_rounds,
                          static_cast<long long>(sort_round_requests(s)), watchdog_cycles(T), mma_wait_cycles(T),
@@ -1249,7 +1332,7 @@ int run_trace_device(bbrt_scene* s, const double* d_o, const double* d_d, long l
     if (rc) return rc;
     GraphLaunch graph;
     if (n < scene_tuning(s).wave_min_rays) {
-        BBRT_CUDA(timed(s, K_TAIL, st, [&] { return bbrt::launch_trace(s->dev, A, st, s->sm_count); }));
+        BBRT_CUDA(timed(s, K_TAIL, st, [&] { return bbrt::launch_rays(s->dev, A, bbrt::WaveArgs(), nullptr, nullptr, n, s->sm_count, st); }));
     } else {
         rc = run_wavefront(s, A, st, graph);
         if (rc) return rc;
@@ -1517,7 +1600,7 @@ BBRT_API int bbrt_intersect(bbrt_scene_t s, const double* origins, const double*
         Q.origins = origins;
         Q.dirs = dirs;
         Q.out = out;
-        BBRT_CUDA(bbrt::launch_query(s->dev, Q, st));
+        BBRT_CUDA((mode == BBRT_QUERY_BVH ? bbrt::launch_query_warp(s->dev, Q, s->sm_count, st) : bbrt::launch_query(s->dev, Q, st)));
         return BBRT_OK;
     }
     const size_t vb = sizeof(double) * 3 * static_cast<size_t>(n);
@@ -1529,7 +1612,7 @@ BBRT_API int bbrt_intersect(bbrt_scene_t s, const double* origins, const double*
     Q.origins = static_cast<const double*>(s->in_o.p);
     Q.dirs = static_cast<const double*>(s->in_d.p);
     Q.out = s->hits.p;
-    BBRT_CUDA(bbrt::launch_query(s->dev, Q, st));
+    BBRT_CUDA((mode == BBRT_QUERY_BVH ? bbrt::launch_query_warp(s->dev, Q, s->sm_count, st) : bbrt::launch_query(s->dev, Q, st)));
     BBRT_CUDA(cudaMemcpyAsync(out, s->hits.p, sizeof(bbrt_hit) * static_cast<size_t>(n), cudaMemcpyDeviceToHost, st));
     BBRT_CUDA(cudaStreamSynchronize(st));
     return BBRT_OK;
@@ -2528,7 +2611,7 @@ BBRT_API int bbrt_trace_batch(const bbrt_scene_t* scenes, int n_scenes, const do
         if (rc) break;
         if (n[k] < scene_tuning(s).wave_min_rays) {
             if (n[k] > 0) {
-                const cudaError_t e = timed(s, K_TAIL, s->stream, [&] { return bbrt::launch_trace(s->dev, A, s->stream, s->sm_count); });
+                const cudaError_t e = timed(s, K_TAIL, s->stream, [&] { return bbrt::launch_rays(s->dev, A, bbrt::WaveArgs(), nullptr, nullptr, A.n, s->sm_count, s->stream); });
                 if (e != cudaSuccess) rc = fail(BBRT_ERR_CUDA, std::string("bbrt_trace_batch: ") + cudaGetErrorString(e));
             }
             runs[k].s = s;
@@ -2843,7 +2926,7 @@ int build_scene_set(const std::vector<bbrt_scene*>& mem, bbrt_scene_set* set) {
         if ((rc = join_device(S, bb, D.c_block_box))) return rc;
     }
     BBRT_CUDA(cudaStreamSynchronize(S.stream));
-    if ((rc = build_leaf_records(&S))) return rc;
+    if ((rc = build_leaf_tables(&S, nbox, nlink, roots))) return rc;
     BBRT_CUDA(S.stats.ensure(sizeof(long long) * bbrt::ST_COUNT));
     BBRT_CUDA(S.work.ensure(sizeof(unsigned long long)));
     S.tables_uploaded = true;

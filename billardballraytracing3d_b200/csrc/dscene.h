@@ -36,7 +36,26 @@ struct DScene {
     // without cull tables), then its patch index (or ~triangle index) and its
     // object index, both as int bits.
     const float4* leaf_rec = nullptr;
-    int smem_nodes = 0;                    // nodes [0, smem_nodes) staged in shared memory
+    // The tree's leaves for queries that look them up instead of walking
+    // (ray_warp.cu), in depth-first (left before right) order, a scene set's
+    // members one after the other:
+    //   leaf_box  [n_leaves][6] FP64 box;  leaf_node [n_leaves] two float4: FP32
+    //   box, first slot and slot count (int bits)
+    //   leaf_rank [n_leaves][8] place in the depth-first order of a ray whose
+    //   1/d is negative on the axes in the octant's bits
+    //   cut_rec   the largest subtrees of at most 32 leaves, two float4 each:
+    //   FP32 box, first leaf and leaf count; cut_box their FP64 boxes
+    //   m_cut     first cut of each member ({0, count} for one scene)
+    // leaf_lists = 0: not usable (a box beyond the FP32 test's range, or a tree
+    // so deep that a walk could overflow its stack).
+    int leaf_lists = 0;
+    const double* leaf_box = nullptr;
+    const float4* leaf_node = nullptr;
+    const int* leaf_rank = nullptr;
+    const float4* cut_rec = nullptr;
+    const double* cut_box = nullptr;
+    const int* m_cut = nullptr;
+    int smem_nodes = 0;                    // nodes [0, smem_nodes) staged in shared memory (k_advance)
     // FP32 copies of the node boxes (nearest rounding) for the FP32 node
     // test, and per axis a bound on |coordinate| over every node box (FP32,
     // rounded up, at least 2^-60); node_f32_ok = 0 when a bound exceeds 2^40

@@ -560,6 +560,32 @@ __device__ __forceinline__ void flush_stats(const TraceArgs& A, const Ctr& ctr, 
     for (int k = 0; k < BBRT_RAY_STATUS_COUNT; ++k) warp_add(A.stats + ST_HIST0 + k, t.hist[k]);
 }
 
+// A query's outcome as the caller's record.
+__device__ __forceinline__ void write_hit(bbrt_hit* out, const QHit& r) {
+    bbrt_hit w;
+    w.t = 0.0;
+    for (int k = 0; k < 3; ++k) { w.point[k] = 0.0; w.normal[k] = 0.0; }
+    w.uv[0] = w.uv[1] = 0.0;
+    w.object = -1;
+    w.status = 0;
+    w.err_object = -1;
+    w.pad_ = 0;
+    w.err_value[0] = w.err_value[1] = 0.0;
+    if (r.err) {
+        w.status = r.err;
+        w.err_object = r.obj;
+        w.err_value[0] = r.ev0;
+        w.err_value[1] = r.ev1;
+    } else if (r.obj >= 0) {
+        w.t = r.t;
+        w.point[0] = r.p.x; w.point[1] = r.p.y; w.point[2] = r.p.z;
+        w.normal[0] = r.n.x; w.normal[1] = r.n.y; w.normal[2] = r.n.z;
+        w.uv[0] = r.u; w.uv[1] = r.v;
+        w.object = r.obj;
+    }
+    *out = w;
+}
+
 // ---- wavefront form: advance rays until they need a Newton solve ----------
 
 __device__ __forceinline__ void save_ray(const WaveArgs& W, long long i, const RayCtx& r, int nres) {
@@ -635,7 +661,7 @@ __device__ __forceinline__ void stage1_tri(const double* __restrict__ X, const d
     if (hit) best.consider(t, (i * nc + j) * 6 + step);
 }
 
-// ---- warp-cooperative stage 1 (used by k_advance and the warp-per-ray tail) ----
+// ---- warp-cooperative stage 1 (used by k_advance and the warp-per-ray kernels) ----
 
 constexpr unsigned kFull = 0xffffffffu;
 

@@ -2,10 +2,10 @@
 // and the bounce loop with reflection and nudge, all in exact FP64.
 //
 // Compiled with -fmad=false: every FP64 decision equals the reference's
-// (see exact.cuh).  Work distribution: one thread per ray, persistent
-// blocks that pull 32-ray batches from a global counter, so warps whose rays
-// finish early (escape on the first query) take new rays instead of idling
-// while a long multi-bounce ray in another warp keeps bouncing.
+// (see exact.cuh).  The wavefront's Newton kernels, its round control, the
+// per-thread tail, single queries by brute force or on one object, and the
+// drivers' ray generation and reductions; rounds are in advance.cu, warp-per-ray
+// traces and queries in ray_warp.cu.
 //
 // Reference (manuelarturosantana/BillardBallRayTracing3D):
 //   RayTracingDriver::trace_ray   include/RayTracingDriver.hpp:172-242
@@ -24,33 +24,9 @@
 
 namespace bbrt {
 
-// Fused per-ray kernel (small batches): warps pull 32-ray batches until none are left.
-__global__ void __launch_bounds__(128) k_trace(DScene S, TraceArgs A) {
-    Counters ctr;
-    RayTally tally;
-    const int lane = threadIdx.x & 31;
-    while (true) {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(A.work_counter, 32ULL);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= static_cast<unsigned long long>(A.n)) break;
-        const long long i = static_cast<long long>(base) + lane;
-        if (i < A.n) {
-            init_outputs(A, i);
-            RayCtx r = start_ray(A, i);
-            Counters c1;
-            run_ray(S, A, i, r, c1, tally.queries);
-            add_ray_work(A, i, c1);
-            ctr.node_tests += c1.node_tests; ctr.patch_tests += c1.patch_tests; ctr.cell_tests += c1.cell_tests;
-            ctr.tri_tests += c1.tri_tests; ctr.newton_iters += c1.newton_iters; ctr.off_patch += c1.off_patch;
-            finish_ray(A, i, r);
-            tally.bounces += r.bounces;
-            tally.hist[r.status]++;
-        }
-    }
-    flush_stats(A, ctr, tally, true);
-}
-
+cudaError_t launch_rays(const DScene& S, const TraceArgs& A, const WaveArgs& W, const NewtonRequest* reqs, const int* rays,
+                        long long n, int sm_count, cudaStream_t stream);
+cudaError_t rays_prepare();
 
 // Newton on patch pidx in the scene's precision mode.
 __device__ __forceinline__ int newton_mode(const DScene& S, int pidx, const V3& o, const V3& d, double u, double v,
@@ -247,191 +223,7 @@ __global__ void __launch_bounds__(128) k_resume(DScene S, TraceArgs A, WaveArgs 
     flush_stats(A, ctr, tally, true);
 }
 
-// ---- warp-per-ray form: 32 lanes cooperate on one ray ----------------------
-//
-// Used for the last rays of a wavefront trace, where too few rays are left
-// to fill the GPU and one lane per ray would run each ray's long chain of
-// dependent queries alone.  Traversal, bookkeeping and Newton run on every
-// lane with identical values (the warp stays converged); the stage-1 box and
-// triangle tests of a patch are split over the lanes and the winner is the
-// (t, key) minimum over the warp, which is what the reference's ordered loop
-// keeps for finite t.  Non-finite rays take the ordered per-lane loop.
-
-// BVH::intersect for one ray with a whole warp (every lane returns the same result).
-// Nodes [0, staged) are read from the shared-memory copy (sbox, slink).
-template <class Ctr>
-__device__ QHit warp_bvh_query(const DScene& S, const V3& o, const V3& d, int cull_flag, int lane, Ctr& ctr,
-                               const double* sbox, const float* sbox32, const int* slink, int staged, bool node_f32,
-                               bool off_patch_miss, int member) {
-    QHit best;
-    best.obj = -1;
-    best.err = 0;
-    best.t = CUDART_INF;
-    const double inv[3] = { 1.0 / d.x, 1.0 / d.y, 1.0 / d.z };
-    const bool neg[3] = { inv[0] < 0.0, inv[1] < 0.0, inv[2] < 0.0 };
-    const bool use_cull = cull_ok(S, member, cull_flag, o, d);
-    bool node32 = node_f32 && finite3(o) && finite3(d);
-    CullRay cr;
-    if (use_cull || node32) cr = make_cull_ray(S, member, o, d);
-    float e32 = 0.0f;
-    if (node32) node32 = node_margin(S, cr, e32);
-    double best_t = CUDART_INF;
-    int stack[64];
-    int sp = 0;
-    stack[sp++] = root_node(S, member);
-    while (sp > 0) {
-        const int idx = stack[--sp];
-        if (lane == 0) ++ctr.node_tests;
-        const bool in_smem = idx < staged;
-        // FP32 node test where it decides (the staged copy then holds FP32 boxes)
-        int dec = -1;
-        if (node32) dec = node_box_f32(in_smem ? sbox32 + 6 * idx : S.node_box32 + 6LL * idx, cr, e32, best_t);
-        if (dec < 0) {
-            if (node32 && lane == 0) ++ctr.node_f64;
-            dec = ray_box_exact(o, inv, in_smem && !node_f32 ? sbox + 6 * idx : S.node_box + 6LL * idx, best_t);
-        }
-        if (!dec) continue;
-        const int* link = in_smem ? slink + 4 * idx : S.node_link + 4LL * idx;
-        if (link[1] < 0) {
-            const int start = link[0], count = link[2];
-            // lane k takes slot k's box; only the objects that pass are tried, in order
-            for (int k0 = 0; k0 < count; k0 += 32) {
-              LeafRec rec;
-              bool try_it = false, culled = false;
-              if (k0 + lane < count) {
-                  rec = load_leaf(S, start + k0 + lane);
-                  try_it = rec.sub() < 0 || !use_cull || cull_leaf(rec, cr);
-                  culled = !try_it;
-              }
-              if constexpr (Ctr::kOn) {
-                  const int nc = __popc(__ballot_sync(kFull, culled));
-                  if (lane == 0) {
-                      ctr.patch_tests += nc;
-                      ctr.cell_tests += nc;
-                  }
-              }
-              for (unsigned todo = __ballot_sync(kFull, try_it); todo; todo &= todo - 1) {
-                const int src = __ffs(todo) - 1;
-                const int obj = __shfl_sync(kFull, rec.obj(), src);
-                const int sub = __shfl_sync(kFull, rec.sub(), src);
-                QHit h;
-                h.err = 0;
-                h.ev0 = h.ev1 = 0.0;
-                int r = 0;
-                if (sub >= 0) {
-                    const int pidx = sub;
-                    const Stage1 s1 = warp_patch_stage1(S, pidx, o, d, use_cull, cr, lane, ctr);
-                    if (s1.have) {
-                        double u0, v0;
-                        key_to_uv(S, s1.key, u0, v0);
-                        long long it = 0;
-                        // One ray per warp: the solve is latency-bound, so
-                        // when every patch axis has at most 8 nodes each
-                        // 8-lane group evaluates it with one node row per lane
-                        // (the same result bit for bit; all four groups agree).
-                        if (S.max_nodes <= kGroup) r = grp_newton_exact(S, pidx, o, d, u0, v0, s1.t, h, it, make_grp());
-                        else r = newton_exact(S, pidx, o, d, u0, v0, s1.t, h, it);
-                        if (lane == 0) ctr.newton_iters += it;
-                    }
-                } else {
-                    CountersT<false> dummy;
-                    r = triangle_intersect(S, ~sub, o, d, h, dummy);
-                }
-                if (off_patch_miss && h.err == BBRT_RAY_NEWTON_DOMAIN) {
-                    if (lane == 0) ++ctr.off_patch;
-                    continue;
-                }
-                if (h.err) {
-                    h.obj = obj;
-                    return h;
-                }
-                if (r && h.t < best_t) {
-                    best_t = h.t;
-                    best = h;
-                    best.obj = obj;
-                }
-              }
-            }
-            continue;
-        }
-        if (sp + 2 > 64) {
-            best.err = BBRT_RAY_STACK_OVERFLOW;
-            best.obj = -1;
-            return best;
-        }
-        const int left = link[0], right = link[1];
-        if (neg[link[3]]) { stack[sp++] = left; stack[sp++] = right; }
-        else              { stack[sp++] = right; stack[sp++] = left; }
-    }
-    return best;
-}
-
-// Finishes rays from their saved state, one warp per ray.
-// MINB blocks of 128 threads per SM requested from the register allocator;
-// the first S.smem_nodes BVH nodes are staged in shared memory.
-template <int MINB, bool STATS>
-__global__ void __launch_bounds__(128, MINB) k_resume_warp(DScene S, TraceArgs A, WaveArgs W,
-                                                           const NewtonRequest* reqs, const int* rays, long long n) {
-    extern __shared__ __align__(16) double smem_tail[];
-    // staged nodes: FP64 boxes, or FP32 boxes with the FP32 node test, then links
-    const bool f32 = W.node_f32 != 0;
-    double* sbox = smem_tail;
-    float* sbox32 = reinterpret_cast<float*>(smem_tail);
-    int* slink = f32 ? reinterpret_cast<int*>(sbox32 + 6 * S.smem_nodes)
-                     : reinterpret_cast<int*>(smem_tail + 6 * S.smem_nodes);
-    if (f32) {
-        for (int k = threadIdx.x; k < 6 * S.smem_nodes; k += blockDim.x) sbox32[k] = S.node_box32[k];
-    } else {
-        for (int k = threadIdx.x; k < 6 * S.smem_nodes; k += blockDim.x) sbox[k] = S.node_box[k];
-    }
-    for (int k = threadIdx.x; k < 4 * S.smem_nodes; k += blockDim.x) slink[k] = S.node_link[k];
-    __syncthreads();
-    if (W.count_dev) n = *W.count_dev;
-    const int lane = threadIdx.x & 31;
-    const long long warp = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-    const long long n_warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-    CountersT<STATS> ctr;
-    RayTallyT<STATS> tally;
-    // The tail's time is that of its slowest warp: rays are handed out one
-    // at a time from a counter, so a warp that drew a long chain takes no
-    // further rays while others do (a fixed stride when no counter is given).
-    unsigned int* next = W.counters ? W.counters + (reqs ? kWcTailNext : kWcOvfNext) : nullptr;
-    auto take = [&](long long fixed) -> long long {
-        if (!next) return fixed;
-        unsigned int v = 0;
-        if (lane == 0) v = atomicAdd(next, 1u);
-        return static_cast<long long>(__shfl_sync(0xffffffffu, v, 0));
-    };
-    for (long long slot = take(warp); slot < n; slot = take(slot + n_warps)) {
-        const long long i = reqs ? reqs[slot].ray : rays[slot];
-        int nres;
-        RayCtx r = load_ray(A, W, i, nres);
-        CountersT<STATS> c1;
-        while (r.status < 0) {
-            if (r.bounces >= A.max_bounces) { r.status = BBRT_RAY_MAX_BOUNCES; break; }
-            if (lane == 0) ++tally.queries;
-            const QHit h = warp_bvh_query(S, r.o, r.d, A.cull, lane, c1, sbox, sbox32, slink, S.smem_nodes, f32,
-                                          A.off_patch_miss != 0, r.member);
-            if (!step_ray(S, A, i, r, h, lane == 0)) break;
-        }
-        if (lane == 0) {
-            add_ray_work(A, i, c1);
-            finish_ray(A, i, r);
-            tally.bounces += r.bounces;
-            tally.hist[r.status]++;
-        }
-        ctr.node_tests += c1.node_tests;
-        ctr.patch_tests += c1.patch_tests;
-        ctr.cell_tests += c1.cell_tests;
-        ctr.tri_tests += c1.tri_tests;
-        ctr.newton_iters += c1.newton_iters;
-        ctr.off_patch += c1.off_patch;
-        ctr.node_f64 += c1.node_f64;
-    }
-    flush_stats(A, ctr, tally, true);
-}
-
-// One query per ray: BVH, brute force over all objects, or one object.
+// One query per thread: brute force over all objects, or one object.
 __global__ void __launch_bounds__(128) k_query(DScene S, QueryArgs Q) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (i >= Q.n) return;
@@ -447,9 +239,7 @@ __global__ void __launch_bounds__(128) k_query(DScene S, QueryArgs Q) {
     const bool use_cull = cull_ok(S, -1, Q.cull, o, d);
     CullRay cr;
     if (use_cull) cr = make_cull_ray(S, -1, o, d);
-    if (Q.mode == BBRT_QUERY_BVH) {
-        r = bvh_query(S, o, d, Q.cull, ctr);
-    } else if (Q.mode == BBRT_QUERY_BRUTE) {
+    if (Q.mode == BBRT_QUERY_BRUTE) {
         bool have = false;
         for (int k = 0; k < S.n_objects; ++k) {
             QHit h;
@@ -464,48 +254,13 @@ __global__ void __launch_bounds__(128) k_query(DScene S, QueryArgs Q) {
         if (h.err) { r = h; r.obj = Q.object; }
         else if (hit) { r = h; r.obj = Q.object; }
     }
-    bbrt_hit* out = static_cast<bbrt_hit*>(Q.out) + i;
-    bbrt_hit w;
-    w.t = 0.0;
-    for (int k = 0; k < 3; ++k) { w.point[k] = 0.0; w.normal[k] = 0.0; }
-    w.uv[0] = w.uv[1] = 0.0;
-    w.object = -1;
-    w.status = 0;
-    w.err_object = -1;
-    w.pad_ = 0;
-    w.err_value[0] = w.err_value[1] = 0.0;
-    if (r.err) {
-        w.status = r.err;
-        w.err_object = r.obj;
-        w.err_value[0] = r.ev0;
-        w.err_value[1] = r.ev1;
-    } else if (r.obj >= 0) {
-        w.t = r.t;
-        w.point[0] = r.p.x; w.point[1] = r.p.y; w.point[2] = r.p.z;
-        w.normal[0] = r.n.x; w.normal[1] = r.n.y; w.normal[2] = r.n.z;
-        w.uv[0] = r.u; w.uv[1] = r.v;
-        w.object = r.obj;
-    }
-    *out = w;
+    write_hit(static_cast<bbrt_hit*>(Q.out) + i, r);
 }
 
 // ---- host launchers -------------------------------------------------------
-cudaError_t launch_trace(const DScene& S, const TraceArgs& A, cudaStream_t stream, int sm_count) {
-    if (A.n <= 0) return cudaSuccess;
-    int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace, 128, 0);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    long long blocks = static_cast<long long>(per_sm) * sm_count;
-    const long long need = (A.n + 127) / 128;
-    if (blocks > need) blocks = need;
-    k_trace<<<static_cast<unsigned>(blocks), 128, 0, stream>>>(S, A);
-    return cudaGetLastError();
-}
-
 // ---- allocation-free trace (bbrt_trace_noalloc) ----------------------------
 //
-// The fused trace kernel's scratch — its ray counter, its statistics block
+// The trace kernel's scratch — its ray counter, its statistics block
 // and per-object hit counters — lives in this file-scope device array
 // instead of memory allocated per scene or per call: word 0 is the counter,
 // words [1, 1 + ST_COUNT) the statistics, words [kNoAllocHeader,
@@ -539,7 +294,7 @@ cudaError_t noalloc_scratch(unsigned long long** out) {
 }
 
 // Loads, on the current device, everything bbrt_trace_noalloc needs from this
-// module: the scratch array's address and the fused trace kernel.  Under lazy
+// module: the scratch array's address and the warp-per-ray kernels.  Under lazy
 // module loading the first use of either would otherwise load the module
 // (which allocates device memory, the array included) inside the first
 // allocation-free call; bbrt_scene_upload calls this instead.
@@ -547,11 +302,10 @@ cudaError_t noalloc_prepare() {
     unsigned long long* p = nullptr;
     cudaError_t e = noalloc_scratch(&p);
     if (e != cudaSuccess) return e;
-    cudaFuncAttributes fa;
-    return cudaFuncGetAttributes(&fa, k_trace);
+    return rays_prepare();
 }
 
-// The fused trace kernel with its scratch in g_noalloc_scratch.  Clears the
+// The warp-per-ray trace with its scratch in g_noalloc_scratch.  Clears the
 // words this call uses first, then traces; hit counters (when asked for) are
 // copied to the caller's device array and the statistics to `host_stats`.
 cudaError_t launch_trace_noalloc(const DScene& S, TraceArgs A, bool count_hits, long long* hit_counts_out,
@@ -565,7 +319,7 @@ cudaError_t launch_trace_noalloc(const DScene& S, TraceArgs A, bool count_hits, 
     A.work_counter = scratch;
     A.stats = reinterpret_cast<long long*>(scratch + 1);
     A.hit_counts = count_hits ? scratch + kNoAllocHeader : nullptr;
-    e = launch_trace(S, A, stream, sm_count);
+    e = launch_rays(S, A, WaveArgs(), nullptr, nullptr, A.n, sm_count, stream);
     if (e != cudaSuccess) return e;
     if (count_hits) {
         e = cudaMemcpyAsync(hit_counts_out, scratch + kNoAllocHeader, sizeof(long long) * S.n_objects,
@@ -660,52 +414,6 @@ cudaError_t launch_resume(const DScene& S, const TraceArgs& A, const WaveArgs& W
     if (n <= 0) return cudaSuccess;
     k_resume<<<static_cast<unsigned>((n + 127) / 128), 128, 0, stream>>>(S, A, W, reqs, rays, n);
     return cudaGetLastError();
-}
-
-template <int MINB, bool STATS>
-static cudaError_t launch_resume_warp_stats(const DScene& S, const TraceArgs& A, const WaveArgs& W,
-                                            const NewtonRequest* reqs, const int* rays, long long n, int sm_count,
-                                            int max_smem_nodes, cudaStream_t stream) {
-    DScene Sl = S;
-    if (Sl.smem_nodes > max_smem_nodes) Sl.smem_nodes = max_smem_nodes;
-    const size_t smem = static_cast<size_t>(Sl.smem_nodes) *
-                        ((W.node_f32 ? 6 * sizeof(float) : 6 * sizeof(double)) + 4 * sizeof(int));
-    cudaError_t e = cudaFuncSetAttribute(k_resume_warp<MINB, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resume_warp<MINB, STATS>, 128, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    long long blocks = static_cast<long long>(per_sm) * sm_count;
-    const long long need = (n + 3) / 4;   // four warps (rays) per block
-    if (blocks > need) blocks = need;
-    k_resume_warp<MINB, STATS><<<static_cast<unsigned>(blocks), 128, smem, stream>>>(Sl, A, W, reqs, rays, n);
-    return cudaGetLastError();
-}
-
-// The statistics-free instance unless the call collects statistics or a per-ray work profile.
-template <int MINB>
-static cudaError_t launch_resume_warp_shape(const DScene& S, const TraceArgs& A, const WaveArgs& W,
-                                            const NewtonRequest* reqs, const int* rays, long long n, int sm_count,
-                                            int max_smem_nodes, cudaStream_t stream) {
-    if (A.stats || A.ray_work)
-        return launch_resume_warp_stats<MINB, true>(S, A, W, reqs, rays, n, sm_count, max_smem_nodes, stream);
-    return launch_resume_warp_stats<MINB, false>(S, A, W, reqs, rays, n, sm_count, max_smem_nodes, stream);
-}
-
-// Tail launch shapes (blocks of 128 threads per SM, BVH nodes staged in
-// shared memory): 0 = 3 blocks, none staged; 1 = 4 blocks, 768 nodes;
-// 2 = 3 blocks, 1024 nodes; 3 = 2 blocks, 1536 nodes.
-cudaError_t launch_resume_warp(const DScene& S, const TraceArgs& A, const WaveArgs& W, const NewtonRequest* reqs,
-                               const int* rays, long long n, int sm_count, int shape, cudaStream_t stream) {
-    if (n <= 0) return cudaSuccess;
-    switch (shape) {
-        case 1: return launch_resume_warp_shape<4>(S, A, W, reqs, rays, n, sm_count, 768, stream);
-        case 2: return launch_resume_warp_shape<3>(S, A, W, reqs, rays, n, sm_count, 1024, stream);
-        case 3: return launch_resume_warp_shape<2>(S, A, W, reqs, rays, n, sm_count, 1536, stream);
-        default: return launch_resume_warp_shape<3>(S, A, W, reqs, rays, n, sm_count, 0, stream);
-    }
 }
 
 // Leaf records (DScene::leaf_rec) from the leaf order and the cull tables: one
