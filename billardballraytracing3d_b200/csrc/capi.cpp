@@ -751,7 +751,8 @@ cudaError_t timed(bbrt_scene* s, int kind, cudaStream_t st, F&& launch) {
 // smaller ones (and the last few rays of a wavefront) run one ray per thread
 // to the end.
 struct Tuning {
-    long long wave_min_rays = 8192;   // smaller batches: one ray per thread to the end
+    long long wave_min_rays = 8192;   // smaller batches: one ray per warp to the end (see wave_min)
+    bool wave_min_set = false;        // ... given by the environment
     long long wave_tail = 4096;       // last requests finished one ray per warp
     int order_rays = 1;               // bucket rays by origin / direction before round 0
     int log_rounds = 0;               // print per-round counts and times to stderr
@@ -775,7 +776,7 @@ struct Tuning {
 const Tuning& tuning() {
     static const Tuning t = [] {
         Tuning v;
-        if (const char* e = std::getenv("BBRT_WAVE_MIN")) v.wave_min_rays = std::atoll(e);
+        if (const char* e = std::getenv("BBRT_WAVE_MIN")) { v.wave_min_rays = std::atoll(e); v.wave_min_set = true; }
         if (const char* e = std::getenv("BBRT_WAVE_TAIL")) v.wave_tail = std::atoll(e);
         if (const char* e = std::getenv("BBRT_ORDER_RAYS")) v.order_rays = std::atoi(e);
         if (const char* e = std::getenv("BBRT_LOG_ROUNDS")) v.log_rounds = std::atoi(e);
@@ -831,6 +832,21 @@ bbrt_tuning scene_tuning(const bbrt_scene* s) {
     t.watchdog_cycles = 0;
     t.mma_wait_cycles = 0;
     return t;
+}
+
+// Batches of at least this many rays run as a wavefront, smaller ones a warp
+// per ray.  A schedule that was set or autotuned says; else, for the FP64 form,
+// 32,768: warp per ray against wavefront, us, at 16,384 / 32,768 / 65,536 rays:
+// tetrahedron 360 / 581 / 1082 against 525 / 611 / 832, ellipsoids 190 / 319 /
+// 589 against 308 / 518 / 635, two spheres 180 / 309 / 547 against 226 / 360 /
+// 416.  The split and learned forms keep 8,192, and so does sample recording:
+// their rounds solve (or record) what the warp-per-ray form would solve in FP64
+// (or not record).
+long long wave_min(const bbrt_scene* s) {
+    if (s->tune_set) return s->tune.wave_min_rays;
+    const bool plain = s->dev.precision == BBRT_PREC_FP64 && !s->rec_samples &&
+                       !(s->host.cfg.guess == BBRT_GUESS_LEARNED && s->guess.trained);
+    return plain && !tuning().wave_min_set ? 32768 : tuning().wave_min_rays;
 }
 
 // The k_advance watchdog and the tensor-core wait bound of a schedule
@@ -1331,7 +1347,7 @@ int run_trace_device(bbrt_scene* s, const double* d_o, const double* d_d, long l
     int rc = prepare_trace(s, d_o, d_d, n, max_bounces, out_dev, hit_counts, count_from, st, want_stats, A);
     if (rc) return rc;
     GraphLaunch graph;
-    if (n < scene_tuning(s).wave_min_rays) {
+    if (n < wave_min(s)) {
         BBRT_CUDA(timed(s, K_TAIL, st, [&] { return bbrt::launch_rays(s->dev, A, bbrt::WaveArgs(), nullptr, nullptr, n, s->sm_count, st); }));
     } else {
         rc = run_wavefront(s, A, st, graph);
@@ -1343,7 +1359,7 @@ int run_trace_device(bbrt_scene* s, const double* d_o, const double* d_d, long l
         BBRT_CUDA(cudaEventSynchronize(s->ev[1]));
         rc = check_wave_graph(s, graph);
     }
-    if (!rc && n >= scene_tuning(s).wave_min_rays) rc = check_guess_waits(s, st);
+    if (!rc && n >= wave_min(s)) rc = check_guess_waits(s, st);
     return rc;
 }
 
@@ -2609,7 +2625,7 @@ BBRT_API int bbrt_trace_batch(const bbrt_scene_t* scenes, int n_scenes, const do
         rc = prepare_trace(s, origins[k], dirs[k], n[k], max_bounces, outs ? &outs[k] : nullptr, nullptr, 1, s->stream,
                            want, A);
         if (rc) break;
-        if (n[k] < scene_tuning(s).wave_min_rays) {
+        if (n[k] < wave_min(s)) {
             if (n[k] > 0) {
                 const cudaError_t e = timed(s, K_TAIL, s->stream, [&] { return bbrt::launch_rays(s->dev, A, bbrt::WaveArgs(), nullptr, nullptr, A.n, s->sm_count, s->stream); });
                 if (e != cudaSuccess) rc = fail(BBRT_ERR_CUDA, std::string("bbrt_trace_batch: ") + cudaGetErrorString(e));
@@ -2635,7 +2651,7 @@ BBRT_API int bbrt_trace_batch(const bbrt_scene_t* scenes, int n_scenes, const do
         }
     }
     for (int k = 0; k < n_scenes && !rc; ++k) {
-        if (runs[k].s && n[k] >= scene_tuning(scenes[k]).wave_min_rays) rc = runs[k].finish();
+        if (runs[k].s && n[k] >= wave_min(scenes[k])) rc = runs[k].finish();
         if (!rc) rc = complete_trace(scenes[k], scenes[k]->stream, want, hs[k].data(), nullptr);
         if (!rc && scenes[k]->stream != bs) {
             cudaEvent_t e = scenes[k]->ev[1];
@@ -2649,7 +2665,7 @@ BBRT_API int bbrt_trace_batch(const bbrt_scene_t* scenes, int n_scenes, const do
     for (int k = 0; k < n_scenes && !rc; ++k)
         if (runs[k].graph.on) rc = check_wave_graph(scenes[k], runs[k].graph);
     for (int k = 0; k < n_scenes && !rc; ++k)
-        if (n[k] >= scene_tuning(scenes[k]).wave_min_rays) rc = check_guess_waits(scenes[k], scenes[k]->stream);
+        if (n[k] >= wave_min(scenes[k])) rc = check_guess_waits(scenes[k], scenes[k]->stream);
     if (!rc && batch_ms) {
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, start, end);

@@ -20,12 +20,11 @@
 //   3. the leaves' slots, one per lane: the patches whose box the ray meets;
 //   4. stage 1 of all of those at once: block boxes, cell boxes and triangles
 //      as compacted work lists;
-//   5. Newton solves of the stage-1 hits, four at a time by 8-lane groups;
-//   6. the results taken in order, a leaf's box tested again with the best t
-//      found before it, so that what the reference would not have visited
-//      (behind a nearer hit) changes nothing.
-// Work behind the first hit is wasted, but a query is a handful of dependent
-// steps instead of one per node, box level and solve.
+//   5. the stage-1 hits in order, a leaf's box tested again with the best t found
+//      before it, so that what the reference would not have visited (behind a
+//      nearer hit) changes nothing; Newton by the whole warp.
+// Stage 1 behind the first hit is wasted, but a query is a handful of dependent
+// steps instead of one per node and box level.
 //
 // Reference (manuelarturosantana/BillardBallRayTracing3D):
 //   RayTracingDriver::trace_ray   include/RayTracingDriver.hpp:172-242
@@ -37,15 +36,19 @@
 #include <algorithm>
 
 #include "trace_common.cuh"
-#include "newton_group.cuh"
 
 namespace bbrt {
 namespace {
 
 constexpr int kWarps = 4;           // warps per block
+// Blocks per SM asked of the register allocator: 3 leaves 168 registers, 4 (128,
+// three times the spills) measured slower: 4,096 tetrahedron rays 171 against
+// 154 us, 96 queries 64 against 55 us.
+constexpr int kMinBlocks = 3;
 constexpr int kLeafCap = 64;        // leaves one query may visit here (more: warp_bvh_query)
 constexpr int kSlotCap = 256;       // ... and their slots
 constexpr int kListCap = 96;        // blocks and cells waiting to be tested
+constexpr int kAxis = 8;            // nodes per axis of warp_newton
 
 // One warp's shared memory.
 struct RayWork {
@@ -55,6 +58,8 @@ struct RayWork {
     unsigned char slot_leaf[kSlotCap];    // position of a slot's leaf in order[]
     int sub[32], obj[32], leaf_pos[32];   // candidates: patch or ~triangle, object, position in order[]
     int blk[kListCap], cell[kListCap];    // candidate << 24 | block or cell
+    // Newton: barycentric basis (u, then v from kAxis on), rows' sums, evaluated fields
+    double basis[2 * kAxis], rows[kAxis * 9], eval[9];
 };
 
 // node_box_f32 on a record's box.
@@ -102,7 +107,7 @@ __device__ QHit warp_bvh_query(const DScene& S, const V3& o, const V3& d, int cu
                         double u0, v0;
                         key_to_uv(S, s1.key, u0, v0);
                         long long it = 0;
-                        r = newton_exact(S, sub, o, d, u0, v0, s1.t, h, it);
+                        r = newton_exact_j<0>(S, sub, o, d, u0, v0, s1.t, h, it);
                         if (lane == 0) ctr.newton_iters += it;
                     }
                 } else {
@@ -135,6 +140,104 @@ __device__ QHit warp_bvh_query(const DScene& S, const V3& o, const V3& d, int cu
         else              { stack[sp++] = right; stack[sp++] = left; }
     }
     return best;
+}
+
+// Fields first[0] .. first[0] + 2 and so on (NF of them, in threes) of a patch at
+// the basis in w.basis, into w.eval: a lane forms a row's sum over j of one
+// field, then a lane per field adds the rows in order, skipping rows whose
+// basis is 0 (eval_fields' sums in eval_fields' order).
+template <int NF>
+__device__ __forceinline__ void warp_eval(const double* __restrict__ F, int I, int J, RayWork& w, int lane) {
+    for (int p = lane; p < I * NF; p += 32) {
+        const int i = p / NF, f = p - i * NF;
+        const double* row = F + static_cast<long long>(i) * J * 12 + (NF == 6 && f >= 3 ? f + 6 : f);
+        double s = 0.0;
+        if (w.basis[i] != 0.0)
+            for (int j = 0; j < J; ++j) s += w.basis[kAxis + j] * row[j * 12];
+        w.rows[p] = s;
+    }
+    __syncwarp();
+    if (lane < NF) {
+        double e = 0.0;
+        for (int i = 0; i < I; ++i) {
+            const double li = w.basis[i];
+            if (li != 0.0) e += li * w.rows[i * NF + lane];
+        }
+        w.eval[lane] = e;
+    }
+    __syncwarp();
+}
+
+// Both axes' barycentric bases (basis_1d) into w.basis: lanes 0-7 of each
+// half-warp take the u nodes, lanes 8-15 the v nodes.
+// `node`, `weight`: the lane's own (of N on its axis).
+__device__ __forceinline__ void warp_basis(double node, double weight, int N, double x, RayWork& w, int lane) {
+    const int k = lane & (kAxis - 1), base = lane & kAxis;
+    const bool mine = k < N;
+    const double gap = mine ? x - node : 1.0;
+    const unsigned on = __ballot_sync(kFull, mine && fabs(gap) < 1.0e-12) >> base & 0xFFu;
+    const double li = mine ? weight / gap : 0.0;
+    double denom = 0.0;
+#pragma unroll
+    for (int i = 0; i < kAxis; ++i) {
+        const double x_i = __shfl_sync(kFull, li, base + i);
+        if (i < N) denom += x_i;
+    }
+    const double b = on ? (k == __ffs(on) - 1 ? 1.0 : 0.0) : (mine ? li / denom : 0.0);
+    if (lane < 2 * kAxis) w.basis[lane] = b;
+    __syncwarp();
+}
+
+// newton_exact by the whole warp, for patches of at most 8 nodes per axis: the
+// same operations in the same order, so the same result, on every lane.  A
+// query rarely has more than one solve that counts, so the lanes share one
+// solve (63 row sums of 7 nodes for the nine fields) instead of an 8-lane group
+// each: 8-lane groups spent 126 shuffles an iteration on adding the rows up.
+__device__ __forceinline__ int warp_newton(const DScene& S, int pidx, const V3 o, const V3 d, double u, double v, double t,
+                                           QHit& h, long long& iters, RayWork& w, int lane) {
+    const int I = S.p_dims[2 * pidx], J = S.p_dims[2 * pidx + 1];
+    const double* un = S.p_nodes + S.p_node_off[pidx];   // un[I] vn[J] uw[I] vw[J]
+    const bool v_axis = (lane & kAxis) != 0;
+    const int N = v_axis ? J : I, k = min(lane & (kAxis - 1), N - 1) + (v_axis ? I : 0);
+    const double node = un[k], weight = un[I + J + k];
+    const double* F = S.p_fields + S.p_field_off[pidx];
+    double step = CUDART_INF;
+    for (int it = 0; it < S.newton_max_iters; ++it) {
+        ++iters;
+        warp_basis(node, weight, N, v_axis ? v : u, w, lane);
+        warp_eval<9>(F, I, J, w, lane);
+        double e[9];
+#pragma unroll
+        for (int f = 0; f < 9; ++f) e[f] = w.eval[f];
+        const V3 R = v3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z);
+        const double Fx = e[0] - R.x, Fy = e[1] - R.y, Fz = e[2] - R.z;
+        const double a11 = e[3], a12 = e[6], a13 = -d.x;
+        const double a21 = e[4], a22 = e[7], a23 = -d.y;
+        const double a31 = e[5], a32 = e[8], a33 = -d.z;
+        const double det = a11 * (a22 * a33 - a23 * a32) - a12 * (a21 * a33 - a23 * a31) + a13 * (a21 * a32 - a22 * a31);
+        if (fabs(det) < 1e-14) { h.err = BBRT_RAY_NEWTON_SINGULAR; return 0; }
+        const double d0 = Fx * (a22 * a33 - a23 * a32) - a12 * (Fy * a33 - a23 * Fz) + a13 * (Fy * a32 - a22 * Fz);
+        const double d1 = a11 * (Fy * a33 - a23 * Fz) - Fx * (a21 * a33 - a23 * a31) + a13 * (a21 * Fz - Fy * a31);
+        const double d2 = a11 * (a22 * Fz - Fy * a32) - a12 * (a21 * Fz - Fy * a31) + Fx * (a21 * a32 - a22 * a31);
+        const double x0 = d0 / det, x1 = d1 / det, x2 = d2 / det;
+        u -= x0;
+        v -= x1;
+        t -= x2;
+        step = sqrt(x0 * x0 + x1 * x1 + x2 * x2);
+        if (step < S.newton_tol) break;
+    }
+    if (step >= S.newton_tol) { h.err = BBRT_RAY_NEWTON_NOCONV; h.ev0 = step; return 0; }
+    if (u < -1.0 - 1e-6 || u > 1.0 + 1e-6 || v < -1.0 - 1e-6 || v > 1.0 + 1e-6) {
+        h.err = BBRT_RAY_NEWTON_DOMAIN; h.ev0 = u; h.ev1 = v; return 0;
+    }
+    warp_basis(node, weight, N, v_axis ? v : u, w, lane);
+    warp_eval<6>(F, I, J, w, lane);   // point and normal
+    h.t = t;
+    h.p = v3(w.eval[0], w.eval[1], w.eval[2]);
+    h.n = vnormalize(v3(w.eval[3], w.eval[4], w.eval[5]));
+    h.u = u;
+    h.v = v;
+    return 1;
 }
 
 // Stage 1 of the P candidates in w.sub (patches; triangles are left to the
@@ -355,68 +458,47 @@ __device__ __forceinline__ bool ray_query(const DScene& S, RayWork& w, const V3&
         }
         __syncwarp();
         const Stage1 mine = ray_stage1(S, w, P, o, d, use_cull, cr, lane, ctr);
-        // ---- stage-1 hits (and triangles) in order, four solves at a time
-        unsigned hits = __ballot_sync(kFull, lane < P && (mine.have || w.sub[lane < P ? lane : 0] < 0));
-        while (hits) {
-            const Grp G = make_grp();
-            const int g = lane / kGroup, count = min(4, __popc(hits));
-            const int my = g < count ? nth_bit(hits, g) : -1;
-            const double t0 = __shfl_sync(kFull, mine.t, my < 0 ? 0 : my);
-            const int key = __shfl_sync(kFull, mine.key, my < 0 ? 0 : my);
+        // ---- stage-1 hits (and triangles) in order
+        for (unsigned hits = __ballot_sync(kFull, lane < P && (mine.have || w.sub[lane < P ? lane : 0] < 0)); hits;
+             hits &= hits - 1) {
+            const int c = __ffs(hits) - 1;
+            const int lp = w.leaf_pos[c];
+            if (lp != open) {
+                if (best_t < CUDART_INF && !ray_box_exact(o, inv, S.leaf_box + 6LL * w.order[lp], best_t)) continue;
+                open = lp;
+            }
+            const int sub = w.sub[c];
+            const double t0 = __shfl_sync(kFull, mine.t, c);
+            const int key = __shfl_sync(kFull, mine.key, c);
             QHit h;
             h.err = 0;
             h.ev0 = h.ev1 = 0.0;
-            h.t = h.u = h.v = 0.0;
-            h.p = h.n = v3(0.0, 0.0, 0.0);
-            int r = 0;
-            long long it = 0;
-            if (my >= 0) {
-                const int sub = w.sub[my];
-                if (sub >= 0) {
-                    double u0, v0;
-                    key_to_uv(S, key, u0, v0);
-                    if (S.max_nodes <= kGroup) r = grp_newton_exact(S, sub, o, d, u0, v0, t0, h, it, G);
-                    else r = newton_exact(S, sub, o, d, u0, v0, t0, h, it);
-                } else {
-                    CountersT<false> dummy;
-                    r = triangle_intersect(S, ~sub, o, d, h, dummy);
-                }
+            int r;
+            if (sub >= 0) {
+                double u0, v0;
+                key_to_uv(S, key, u0, v0);
+                long long it = 0;
+                if (S.max_nodes <= kAxis) r = warp_newton(S, sub, o, d, u0, v0, t0, h, it, w, lane);
+                else r = newton_exact_j<0>(S, sub, o, d, u0, v0, t0, h, it);
+                if (lane == 0) ctr.newton_iters += it;
+            } else {
+                CountersT<false> dummy;
+                r = triangle_intersect(S, ~sub, o, d, h, dummy);
             }
-            __syncwarp();
-            for (int k = 0; k < count; ++k, hits &= hits - 1) {
-                const int src = k * kGroup, c = __ffs(hits) - 1;
-                if constexpr (Ctr::kOn) {
-                    const long long its = __shfl_sync(kFull, it, src);
-                    if (lane == 0) ctr.newton_iters += its;
-                }
-                const int lp = w.leaf_pos[c];
-                if (lp != open) {
-                    if (best_t < CUDART_INF && !ray_box_exact(o, inv, S.leaf_box + 6LL * w.order[lp], best_t)) continue;
-                    open = lp;
-                }
-                const int err = __shfl_sync(kFull, h.err, src), rr = __shfl_sync(kFull, r, src);
-                if (off_patch_miss && err == BBRT_RAY_NEWTON_DOMAIN) {
-                    if (lane == 0) ++ctr.off_patch;
-                    continue;
-                }
-                if (err) {
-                    best.err = err;
-                    best.obj = w.obj[c];
-                    best.ev0 = __shfl_sync(kFull, h.ev0, src);
-                    best.ev1 = __shfl_sync(kFull, h.ev1, src);
-                    __syncwarp();
-                    return true;
-                }
-                const double t = __shfl_sync(kFull, h.t, src);
-                if (rr && t < best_t) {
-                    best_t = t;
-                    best.obj = w.obj[c];
-                    best.t = t;
-                    best.p = v3(__shfl_sync(kFull, h.p.x, src), __shfl_sync(kFull, h.p.y, src), __shfl_sync(kFull, h.p.z, src));
-                    best.n = v3(__shfl_sync(kFull, h.n.x, src), __shfl_sync(kFull, h.n.y, src), __shfl_sync(kFull, h.n.z, src));
-                    best.u = __shfl_sync(kFull, h.u, src);
-                    best.v = __shfl_sync(kFull, h.v, src);
-                }
+            if (off_patch_miss && h.err == BBRT_RAY_NEWTON_DOMAIN) {
+                if (lane == 0) ++ctr.off_patch;
+                continue;
+            }
+            if (h.err) {
+                best = h;
+                best.obj = w.obj[c];
+                __syncwarp();
+                return true;
+            }
+            if (r && h.t < best_t) {
+                best_t = h.t;
+                best = h;
+                best.obj = w.obj[c];
             }
         }
         __syncwarp();
@@ -437,7 +519,7 @@ __device__ __forceinline__ QHit any_query(const DScene& S, RayWork& w, const V3&
 // saved rays of `reqs` / `rays`, whose current query starts again.  Rays are
 // handed out one at a time, so a warp that drew a long chain takes no more.
 template <bool STATS>
-__global__ void __launch_bounds__(kWarps * 32, 4) k_rays(DScene S, TraceArgs A, WaveArgs W, const NewtonRequest* reqs,
+__global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_rays(DScene S, TraceArgs A, WaveArgs W, const NewtonRequest* reqs,
                                                          const int* rays, long long n) {
     __shared__ RayWork work[kWarps];
     RayWork& w = work[threadIdx.x >> 5];
@@ -486,7 +568,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) k_rays(DScene S, TraceArgs A, 
 }
 
 // BVH queries, one per warp at a time.
-__global__ void __launch_bounds__(kWarps * 32, 4) k_query_warp(DScene S, QueryArgs Q) {
+__global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_query_warp(DScene S, QueryArgs Q) {
     __shared__ RayWork work[kWarps];
     RayWork& w = work[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;

@@ -431,7 +431,8 @@ typedef struct bbrt_tuning {
     int order_rays;           /* 1 (default): bucket rays by direction and origin before round 0 */
     int warp_tail;            /* 1 (default): the tail one warp per ray, else one thread per ray */
     long long wave_tail;      /* rays still waiting when the tail takes over (4096) */
-    long long wave_min_rays;  /* smaller batches run the fused per-thread kernel (8192) */
+    long long wave_min_rays;  /* smaller batches run one ray per warp to the end (8192; a scene whose schedule
+                                 was never set or autotuned takes 32768 in the plain FP64 form) */
     int graph_rounds;         /* 1 (default): the whole wavefront trace is one CUDA graph launch whose
                                  round loop is a device-side conditional node (no host wait per round;
                                  one graph per argument set, kept for reuse); 0: rounds driven by the host */
