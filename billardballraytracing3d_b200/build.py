@@ -28,6 +28,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_FLAGS = {
     "advance.cu": ["-fmad=false"],
     "ray_warp.cu": ["-fmad=false"],
+    "rounds.cu": ["-fmad=false"],
     "trace_kernels.cu": ["-fmad=false"],
     "scene_compile.cu": ["-fmad=false"],
 }

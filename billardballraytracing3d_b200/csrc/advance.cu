@@ -20,20 +20,21 @@ namespace {
 // What a lane's ray is doing.  Everything from M_FINISH on leaves the working
 // loop for the retire / fetch step.
 enum AdvMode {
-    M_TRAV = 0,      // walking the BVH or the slots of a leaf
-    M_S1 = 1,        // at a patch whose stage 1 is to be run
-    M_S1_DONE = 2,   // stage 1 of that patch finished
-    M_RESOLVE = 3,   // query finished: bounce, escape or error
-    M_FINISH = 4,    // ray finished, its results written
-    M_SUSPEND = 5,   // waiting for a Newton solve
-    M_OVERFLOW = 6,  // more solves than the resolved list holds
-    M_IDLE = 7,      // lane has no ray
-    M_DRAINED = 8    // no runnable ray left
+    M_TRAV = 0,      // walking the BVH
+    M_LEAF = 1,      // at the slots of a leaf
+    M_S1 = 2,        // at a patch whose stage 1 is to be run
+    M_S1_DONE = 3,   // stage 1 of that patch finished
+    M_RESOLVE = 4,   // query finished: bounce, escape or error
+    M_FINISH = 5,    // ray finished, its results written
+    M_SUSPEND = 6,   // waiting for a Newton solve
+    M_OVERFLOW = 7,  // more solves than the resolved list holds
+    M_IDLE = 8,      // lane has no ray
+    M_DRAINED = 9    // no runnable ray left
 };
 
 constexpr int kBlkQueue = 512;    // 32 patches of at most 16 blocks
 constexpr int kCellQueue = 128;   // cells waiting for their triangle tests
-constexpr int kCellFlush = kCellQueue - 32;
+constexpr int kCellFlush = kCellQueue - 64;
 
 // One warp's shared memory: its rays (lane's slot), and the work lists of a
 // batch of stage 1s.
@@ -44,6 +45,7 @@ struct WarpWork {
     unsigned short blk[kBlkQueue];     // passing blocks: lane << 8 | block row << 4 | block column
     unsigned short cell[kCellQueue];   // passing cells: lane << 8 | row << 4 | column
     unsigned char lane_of[32];         // lanes of the batch
+    float e[32];                       // margin of the FP32 node test; negative: nodes tested in FP64
     int cells[32], tris[32];           // box and triangle tests of a lane's patch (statistics)
 };
 static_assert(sizeof(WarpWork) % 16 == 0, "per-warp blocks must keep 16-byte alignment");
@@ -58,18 +60,19 @@ __device__ __forceinline__ CullRay work_cull_ray(const WarpWork& w, int lane) {
 __device__ __forceinline__ V3 work_o(const WarpWork& w, int lane) { return v3(w.od[0][lane], w.od[1][lane], w.od[2][lane]); }
 __device__ __forceinline__ V3 work_d(const WarpWork& w, int lane) { return v3(w.od[3][lane], w.od[4][lane], w.od[5][lane]); }
 
+constexpr int kNone = static_cast<int>(0x80000000u);
+
 // Per-lane state of the query being walked.
 struct AdvState {
-    CullRay cr;          // also the FP32 origin and 1/d of the FP32 node test
-    float e32;           // its margin
     bool use_cull;
-    bool node32;         // node boxes tested in FP32 (node_box_f32)
     unsigned neg;        // bit a: 1/d_a < 0 (the reference's child order)
     double best_t;
     int best_obj;        // -1: no hit yet
     int best_e;          // resolved entry of the best patch hit (or of the failed solve), -1 for a triangle
     int err;
+    int ref;             // node to enter next, known to pass (a reference of DScene::pair_rec), or kNone
     int sp;
+    int untested;        // stack entries below this were tested with a larger best_t, or not at all
     int slot, slot_end;  // leaf slots still to look at
     int obj;             // object of the pending stage 1
     Stage1 s1;
@@ -86,38 +89,47 @@ __device__ __forceinline__ void adv_start_query(const DScene& S, const TraceArgs
                                                 int* stack) {
     q.neg = neg_bit(d.x) | (neg_bit(d.y) << 1) | (neg_bit(d.z) << 2);
     q.use_cull = cull_ok(S, member, A.cull, o, d);
-    q.node32 = W.node_f32 && finite3(o) && finite3(d);
-    if (q.use_cull || q.node32) q.cr = make_cull_ray(S, member, o, d);
-    if (q.node32) q.node32 = node_margin(S, q.cr, q.e32);
-    ww.cr_a[lane] = make_float4(q.cr.ox, q.cr.oy, q.cr.oz, q.cr.delta);
-    ww.cr_b[lane] = make_float4(q.cr.ix, q.cr.iy, q.cr.iz, 0.0f);
+    const bool node32 = W.node_f32 && finite3(o) && finite3(d);
+    float e = -1.0f;
+    if (q.use_cull || node32) {
+        const CullRay cr = make_cull_ray(S, member, o, d);
+        ww.cr_a[lane] = make_float4(cr.ox, cr.oy, cr.oz, cr.delta);
+        ww.cr_b[lane] = make_float4(cr.ix, cr.iy, cr.iz, 0.0f);
+        NodeRay nr;
+        if (node32 && make_node_ray(S, cr, nr)) e = nr.e;
+    }
+    ww.e[lane] = e;
     ww.od[0][lane] = o.x; ww.od[1][lane] = o.y; ww.od[2][lane] = o.z;
     ww.od[3][lane] = d.x; ww.od[4][lane] = d.y; ww.od[5][lane] = d.z;
     q.best_t = CUDART_INF;
     q.best_obj = -1;
     q.best_e = -1;
     q.err = 0;
-    q.sp = 1;
+    q.ref = kNone;
+    q.sp = q.untested = 1;
     q.slot = q.slot_end = 0;
-    stack[0] = root_node(S, member);
+    stack[0] = S.m_ref[member < 0 ? 0 : member];
 }
 
-// One BVH node test: in FP32 where the ray allows it and the FP32 interval
-// decides (node_box_f32), else ray_box_exact.
-template <class Ctr>
-__device__ __forceinline__ bool adv_node_pass(const DScene& S, const WarpWork& ww, int lane, const AdvState& q, int idx,
-                                              const float* sbox32, int staged, Ctr& c) {
-    int dec = -1;
-    if (q.node32) {
-        dec = node_box_f32(idx < staged ? sbox32 + 6 * idx : S.node_box32 + 6LL * idx, q.cr, q.e32, q.best_t);
-        if (dec < 0) ++c.node_f64;
-    }
-    if (dec < 0) {
-        const V3 d = work_d(ww, lane);
-        const double inv[3] = { 1.0 / d.x, 1.0 / d.y, 1.0 / d.z };
-        dec = ray_box_exact(work_o(ww, lane), inv, S.node_box + 6LL * idx, q.best_t);
-    }
-    return dec != 0;
+// The lane's ray of the FP32 node test for its query so far, from its slot:
+// formed anew for each stretch of the walk, so that no register holds it
+// through the stage 1s (e < 0: nodes are tested in FP64).
+__device__ __forceinline__ NodeRay work_node_ray(const WarpWork& w, int lane, double best_t) {
+    const CullRay c = work_cull_ray(w, lane);
+    NodeRay r;
+    r.ix = c.ix; r.iy = c.iy; r.iz = c.iz;
+    r.px = -c.ox * c.ix; r.py = -c.oy * c.iy; r.pz = -c.oz * c.iz;
+    r.e = w.e[lane];
+    r.e2 = 2.0f * r.e;
+    r.set_best(best_t);
+    return r;
+}
+
+// The FP64 node test of a lane's ray.
+__device__ __forceinline__ bool work_box_exact(const WarpWork& w, int lane, const double* box, double best_t) {
+    const V3 d = work_d(w, lane);
+    const double inv[3] = { 1.0 / d.x, 1.0 / d.y, 1.0 / d.z };
+    return ray_box_exact(work_o(w, lane), inv, box, best_t);
 }
 
 // Keeps the traversal state of a query that suspends for a Newton solve (the
@@ -147,7 +159,8 @@ __device__ __forceinline__ bool resume_query(const WaveArgs& W, long long i, Adv
     const int* qi = W.qs_int + i * kQsInt;
     const int sp = qi[0];
     if (sp < 0) return false;
-    q.sp = sp;
+    q.ref = kNone;
+    q.sp = q.untested = sp;
     q.slot = qi[1];
     q.slot_end = qi[2];
     q.best_obj = qi[3];
@@ -204,32 +217,64 @@ __device__ __forceinline__ void batch_stage1(const DScene& S, WarpWork& w, unsig
     __syncwarp();
     const int hi = hl / NB, hj = hl - hi * NB;
     int n_blk = 0;
-    for (int p = 0; p < P; p += 2) {
-        const int c = p + half;
-        const int owner = w.lane_of[c < P ? c : p];
-        const int pidx = __float_as_int(w.cr_b[owner].w);
-        bool pass = c < P && hl < NB2;
-        if (pass) pass = cull_box(S.c_block_box + (static_cast<long long>(pidx) * NB2 + hl) * 6, work_cull_ray(w, owner));
-        const unsigned m = __ballot_sync(kFull, pass);
-        if (pass) w.blk[n_blk + __popc(m & lt)] = static_cast<unsigned short>(owner << 8 | hi << 4 | hj);
-        n_blk += __popc(m);
+    // four patches per half-warp with their boxes loaded together: the loads'
+    // latency, not the tests, is what a batch waits for
+    constexpr int U = 1;
+    for (int p = 0; p < P; p += 2 * U) {
+        int owner[U];
+        float2 b[U][3];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int c = p + 2 * k + half;
+            owner[k] = c < P && hl < NB2 ? w.lane_of[c] : -1;
+            if (owner[k] >= 0) {
+                const int pidx = __float_as_int(w.cr_b[owner[k]].w);
+                const float2* src = reinterpret_cast<const float2*>(S.c_block_box + (static_cast<long long>(pidx) * NB2 + hl) * 6);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) b[k][a] = src[a];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const bool pass = owner[k] >= 0 && cull_box(b[k][0], b[k][1], b[k][2], work_cull_ray(w, owner[k]));
+            const unsigned m = __ballot_sync(kFull, pass);
+            if (pass) w.blk[n_blk + __popc(m & lt)] = static_cast<unsigned short>(owner[k] << 8 | hi << 4 | hj);
+            n_blk += __popc(m);
+        }
     }
     __syncwarp();
     int n_cell = 0;
-    for (int p = 0; p < n_blk; p += 2) {
-        const int c = p + half;
-        const int e = w.blk[c < n_blk ? c : p];
-        const int owner = e >> 8;
-        const int i = ((e >> 4) & 15) * 4 + (hl >> 2), j = (e & 15) * 4 + (hl & 3);
-        bool pass = c < n_blk && i < nc && j < nc;
-        if (STATS && pass) atomicAdd(&w.cells[owner], 1);
-        const int pidx = __float_as_int(w.cr_b[owner].w);
-        if (pass) pass = cull_box(S.c_cell_box + (static_cast<long long>(pidx) * nc * nc + i * nc + j) * 6, work_cull_ray(w, owner));
-        if (STATS && pass) atomicAdd(&w.tris[owner], 6);
-        const unsigned m = __ballot_sync(kFull, pass);
-        if (pass) w.cell[n_cell + __popc(m & lt)] = static_cast<unsigned short>(owner << 8 | i << 4 | j);
-        n_cell += __popc(m);
-        if (n_cell > kCellFlush) {
+    constexpr int V = 1;
+    for (int p = 0; p < n_blk; p += 2 * V) {
+        int entry[V];   // owner << 8 | row << 4 | column, or -1
+        float2 b[V][3];
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const int c = p + 2 * k + half;
+            entry[k] = -1;
+            if (c < n_blk) {
+                const int e = w.blk[c], i = ((e >> 4) & 15) * 4 + (hl >> 2), j = (e & 15) * 4 + (hl & 3);
+                if (i < nc && j < nc) {
+                    entry[k] = (e & ~255) | i << 4 | j;
+                    const int pidx = __float_as_int(w.cr_b[e >> 8].w);
+                    const float2* src = reinterpret_cast<const float2*>(S.c_cell_box +
+                                                                        (static_cast<long long>(pidx) * nc * nc + i * nc + j) * 6);
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) b[k][a] = src[a];
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const int owner = entry[k] >> 8;
+            if (STATS && entry[k] >= 0) atomicAdd(&w.cells[owner], 1);
+            const bool pass = entry[k] >= 0 && cull_box(b[k][0], b[k][1], b[k][2], work_cull_ray(w, owner));
+            if (STATS && pass) atomicAdd(&w.tris[owner], 6);
+            const unsigned m = __ballot_sync(kFull, pass);
+            if (pass) w.cell[n_cell + __popc(m & lt)] = static_cast<unsigned short>(entry[k]);
+            n_cell += __popc(m);
+        }
+        if (n_cell > kCellFlush && p + 2 * V < n_blk) {
             __syncwarp();
             batch_tris<STATS>(S, w, n_cell, lane, mine);
             __syncwarp();
@@ -259,14 +304,11 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
     AdvState q;
     int stack[64];
     const int lane = threadIdx.x & 31;
-    // Shared memory: the first S.smem_nodes BVH nodes (breadth-first order: the
-    // top levels), links then FP32 boxes, and one WarpWork per warp.
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    int4* slink = reinterpret_cast<int4*>(smem_raw);
-    float* sbox32 = reinterpret_cast<float*>(slink + S.smem_nodes);
-    WarpWork& ww = reinterpret_cast<WarpWork*>(smem_raw + ((S.smem_nodes * 40 + 15) & ~15))[threadIdx.x >> 5];
-    for (int k = threadIdx.x; k < 6 * S.smem_nodes; k += blockDim.x) sbox32[k] = S.node_box32[k];
-    for (int k = threadIdx.x; k < S.smem_nodes; k += blockDim.x) slink[k] = reinterpret_cast<const int4*>(S.node_link)[k];
+    // Shared memory: the first S.smem_pairs node records (breadth-first order:
+    // the top levels) and one WarpWork per warp.
+    extern __shared__ __align__(16) float4 spair[];
+    WarpWork& ww = reinterpret_cast<WarpWork*>(spair + 4 * S.smem_pairs)[threadIdx.x >> 5];
+    for (int k = threadIdx.x; k < 4 * S.smem_pairs; k += blockDim.x) spair[k] = S.pair_rec[k];
     __syncthreads();
     const bool flat_ok = S.block_cells == 4 && S.n_blocks_side <= 4;
     // Runnable rays of this round: the host's count, or (graph-launched
@@ -288,7 +330,7 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
     // of SM clock, about 17 s by default) records an error and ends instead
     // of holding the GPU; checked on the first iteration and every 256th
     // after it.  Both exits of the loop are warp-uniform (this vote and the
-    // drained vote at the end of the body); the inner walk ends after at most
+    // drained vote at the end of the body); the inner loops end after at most
     // the nodes and slots of one query per lane.
     const long long t_start = clock64();
     unsigned int iter = 0;
@@ -297,79 +339,124 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
             if (lane == 0) atomicOr(&W.counters[3], 1u);
             break;
         }
-        // ---- walk until half of the lanes with a ray wait for something else
+        // ---- walk, and look through the leaves met, until half of the lanes with
+        // a ray wait for something else
         const int half_alive = __popc(__ballot_sync(kFull, mode < M_IDLE)) >> 1;
-        while (true) {
+        NodeRay nr = work_node_ray(ww, lane, q.best_t);
+        do {
+        while (__popc(__ballot_sync(kFull, mode == M_TRAV)) > half_alive) {
             if (mode == M_TRAV) {
-                if (q.slot < q.slot_end) {
-                    const LeafRec rec = load_leaf(S, q.slot);
-                    if (rec.sub() >= 0) {
-                        // a patch whose box the ray misses ends here (not while samples
-                        // are recorded: its stage-1 miss is a training sample)
-                        if (q.use_cull && !A.samples && !cull_leaf(rec, q.cr)) {
-                            ++cray.patch_tests;
-                            ++cray.cell_tests;
-                            ++q.slot;
-                        } else {
-                            const int obj = rec.obj();
-                            int e = -1;
-                            for (int k = 0; k < nres; ++k)
-                                if (W.res_obj[static_cast<long long>(i) * kResolved + k] == obj) { e = k; break; }
-                            if (e < 0) {
-                                q.obj = obj;
-                                ww.cr_b[lane].w = rec.b.z;
-                                mode = M_S1;
-                            } else {
-                                const long long ei = static_cast<long long>(i) * kResolved + e;
-                                q.err = W.res_err[ei];
-                                if (q.err) {
-                                    q.best_e = e;
-                                    q.best_obj = obj;
-                                    mode = M_RESOLVE;
-                                } else {
-                                    const double t = W.res_data[ei * kResData];
-                                    if (t < q.best_t) {
-                                        q.best_t = t;
-                                        q.best_obj = obj;
-                                        q.best_e = e;
-                                    }
-                                    ++q.slot;
-                                }
-                            }
+                int ref = q.ref;
+                if (ref == kNone && q.sp > 0) {
+                    ref = stack[--q.sp];
+                    if (q.sp < q.untested) {
+                        // pushed before best_t was what it is: its own box again
+                        q.untested = q.sp;
+                        ++cray.node_tests;
+                        const float* b32 = ref >= 0 ? S.node_box32 + 6LL * S.pair_node[ref]
+                                                    : reinterpret_cast<const float*>(S.leaf_node + 2LL * ~ref);
+                        int dec = nr.e >= 0.0f ? node_box_f32(b32, nr) : -1;
+                        if (dec < 0) {
+                            if (nr.e >= 0.0f) ++ctr.node_f64;
+                            dec = work_box_exact(ww, lane, ref >= 0 ? S.node_box + 6LL * S.pair_node[ref] : S.leaf_box + 6LL * ~ref,
+                                                 q.best_t);
                         }
-                    } else {
+                        if (!dec) ref = kNone;
+                    }
+                } else if (ref == kNone) {
+                    mode = M_RESOLVE;
+                }
+                q.ref = kNone;
+                if (ref >= 0) {
+                    // both children (their records side by side); a child that fails now
+                    // would fail when the reference pops it, best_t being no larger then
+                    const float4* rec = ref < S.smem_pairs ? spair + 4 * ref : S.pair_rec + 4LL * ref;
+                    const float4 a = rec[0], b = rec[1], c = rec[2], v = rec[3];
+                    int l = -1, r = -1;
+                    cray.node_tests += 2;
+                    if (nr.e >= 0.0f) {
+                        l = node_box_f32(a.x, a.y, a.z, a.w, b.x, b.y, nr);
+                        r = node_box_f32(b.z, b.w, c.x, c.y, c.z, c.w, nr);
+                        if (l < 0) ++ctr.node_f64;
+                        if (r < 0) ++ctr.node_f64;
+                    }
+                    if ((l | r) < 0) {
+                        const double* box = S.node_box + 6LL * __float_as_int(v.x);
+                        if (l < 0) l = work_box_exact(ww, lane, box, q.best_t);
+                        if (r < 0) r = work_box_exact(ww, lane, box + 6, q.best_t);
+                    }
+                    const bool right_first = (q.neg >> __float_as_int(v.w)) & 1u;
+                    const int lref = __float_as_int(v.y), rref = __float_as_int(v.z);
+                    if (l && r) {
+                        q.ref = right_first ? rref : lref;
+                        stack[q.sp++] = right_first ? lref : rref;   // depth of a median-split tree: at most 25
+                    } else if (l || r) {
+                        q.ref = l ? lref : rref;
+                    }
+                } else if (ref != kNone) {
+                    const float4 b = S.leaf_node[2LL * ~ref + 1];
+                    q.slot = __float_as_int(b.z);
+                    q.slot_end = q.slot + __float_as_int(b.w);
+                    mode = M_LEAF;
+                }
+            }
+        }
+        // ---- leaf slots of every lane at a leaf, each to its next patch whose
+        // box the ray meets
+        while (__ballot_sync(kFull, mode == M_LEAF)) {
+            if (mode == M_LEAF) {
+                if (q.slot >= q.slot_end) {
+                    mode = M_TRAV;
+                } else {
+                    const LeafRec rec = load_leaf(S, q.slot);
+                    if (rec.sub() < 0) {
                         QHit h;
                         if (triangle_intersect(S, ~rec.sub(), work_o(ww, lane), work_d(ww, lane), h, cray) && h.t < q.best_t) {
                             q.best_t = h.t;
+                            nr.set_best(q.best_t);
+                            q.untested = q.sp;
                             q.best_obj = rec.obj();
                             q.best_e = -1;
                         }
                         ++q.slot;
-                    }
-                } else if (q.sp == 0) {
-                    mode = M_RESOLVE;
-                } else {
-                    const int idx = stack[--q.sp];
-                    ++cray.node_tests;
-                    if (adv_node_pass(S, ww, lane, q, idx, sbox32, S.smem_nodes, ctr)) {
-                        const int4 link = idx < S.smem_nodes ? slink[idx] : reinterpret_cast<const int4*>(S.node_link)[idx];
-                        if (link.y < 0) {
-                            q.slot = link.x;
-                            q.slot_end = link.x + link.z;
-                        } else if (q.sp + 2 > 64) {
-                            q.err = BBRT_RAY_STACK_OVERFLOW;
-                            q.best_obj = -1;
-                            mode = M_RESOLVE;
+                    } else if (q.use_cull && !A.samples && !cull_leaf(rec, work_cull_ray(ww, lane))) {
+                        // (while samples are recorded, a missed patch is a training sample)
+                        ++cray.patch_tests;
+                        ++cray.cell_tests;
+                        ++q.slot;
+                    } else {
+                        const int obj = rec.obj();
+                        int e = -1;
+                        for (int k = 0; k < nres; ++k)
+                            if (W.res_obj[static_cast<long long>(i) * kResolved + k] == obj) { e = k; break; }
+                        if (e < 0) {
+                            q.obj = obj;
+                            ww.cr_b[lane].w = rec.b.z;
+                            mode = M_S1;
                         } else {
-                            const bool left_far = (q.neg >> link.w) & 1u;
-                            stack[q.sp++] = left_far ? link.x : link.y;
-                            stack[q.sp++] = left_far ? link.y : link.x;
+                            const long long ei = static_cast<long long>(i) * kResolved + e;
+                            q.err = W.res_err[ei];
+                            if (q.err) {
+                                q.best_e = e;
+                                q.best_obj = obj;
+                                mode = M_RESOLVE;
+                            } else {
+                                const double t = W.res_data[ei * kResData];
+                                if (t < q.best_t) {
+                                    q.best_t = t;
+                                    nr.set_best(t);
+                                    q.untested = q.sp;
+                                    q.best_obj = obj;
+                                    q.best_e = e;
+                                }
+                                ++q.slot;
+                            }
                         }
                     }
                 }
             }
-            if (__popc(__ballot_sync(kFull, mode == M_TRAV)) <= half_alive) break;
         }
+        } while (__popc(__ballot_sync(kFull, mode == M_TRAV)) > half_alive);
         // ---- stage 1 of every waiting lane
         const unsigned pend = __ballot_sync(kFull, mode == M_S1);
         if (pend) {
@@ -418,7 +505,7 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
                 if (A.samples)
                     record_sample(A, 0, work_o(ww, lane), work_d(ww, lane), __float_as_int(ww.cr_b[lane].w), 0.0, 0.0, 0.0);
                 ++q.slot;
-                mode = M_TRAV;
+                mode = M_LEAF;
             } else if (nres >= kResolved) {
                 mode = M_OVERFLOW;
             } else {
@@ -477,10 +564,21 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
         // common case): retire suspended / overflowed / finished rays, then
         // let idle lanes fetch the next runnable ray.
         if (__ballot_sync(kFull, mode >= M_FINISH && mode != M_DRAINED) != 0u) {
-            const long long rs = warp_append(&W.counters[0], mode == M_SUSPEND);
-            if (rs >= 0) W.req[rs] = rq;
-            const long long os = warp_append(&W.counters[1], mode == M_OVERFLOW);
-            if (os >= 0) W.overflow[os] = i;
+            // requests, overflows and the rays the free lanes take: three
+            // counters, one round trip
+            const unsigned m_req = __ballot_sync(kFull, mode == M_SUSPEND), m_ovf = __ballot_sync(kFull, mode == M_OVERFLOW);
+            const unsigned m_new = __ballot_sync(kFull, mode >= M_FINISH && mode != M_DRAINED);
+            unsigned at = 0;
+            if (lane < 3) {
+                const int add = __popc(lane == 0 ? m_req : lane == 1 ? m_ovf : m_new);
+                if (add) at = atomicAdd(&W.counters[lane], static_cast<unsigned>(add));
+            }
+            const unsigned before = (1u << lane) - 1u;
+            const unsigned rs = __shfl_sync(kFull, at, 0) + __popc(m_req & before);
+            const unsigned os = __shfl_sync(kFull, at, 1) + __popc(m_ovf & before);
+            const unsigned fs = __shfl_sync(kFull, at, 2) + __popc(m_new & before);
+            if (mode == M_SUSPEND) W.req[rs] = rq;
+            if (mode == M_OVERFLOW) W.overflow[os] = i;
             if (mode == M_SUSPEND || mode == M_OVERFLOW || mode == M_FINISH) {
                 add_ray_work(A, i, cray);
                 ctr.node_tests += cray.node_tests;
@@ -497,7 +595,6 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
                 }
                 mode = M_IDLE;
             }
-            const long long fs = warp_append(&W.counters[2], mode == M_IDLE);
             if (mode == M_IDLE) {
                 if (fs < n_run) {
                     cray = CountersT<STATS>();
@@ -512,15 +609,13 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
                         r = load_ray(A, W, i, nres);
                     }
                     bounces = r.bounces;
-                    bool go = false;
+                    mode = M_TRAV;
                     if (r.status < 0) {
                         adv_start_query(S, A, W, r.member, r.o, r.d, lane, ww, q, stack);
-                        go = (W.runnable != nullptr && resume_query(W, i, q, stack)) || r.bounces < A.max_bounces;
-                        if (!go) r.status = BBRT_RAY_MAX_BOUNCES;
+                        if (W.runnable != nullptr && resume_query(W, i, q, stack)) mode = M_LEAF;
+                        else if (r.bounces >= A.max_bounces) r.status = BBRT_RAY_MAX_BOUNCES;
                     }
-                    if (go) {
-                        mode = M_TRAV;
-                    } else {
+                    if (r.status >= 0) {
                         finish_ray(A, i, r);
                         tally.bounces += r.bounces;
                         tally.hist[r.status]++;
@@ -540,8 +635,7 @@ __global__ void __launch_bounds__(NT, MINB) k_advance(DScene S, TraceArgs A, Wav
 template <int NT, int MINB, bool STATS>
 cudaError_t launch_advance_stats(const DScene& Sl, const TraceArgs& A, const WaveArgs& W, int sm_count,
                                  cudaStream_t stream) {
-    const size_t smem = ((static_cast<size_t>(Sl.smem_nodes) * 40 + 15) & ~static_cast<size_t>(15)) +
-                        (NT / 32) * sizeof(WarpWork);
+    const size_t smem = static_cast<size_t>(Sl.smem_pairs) * 64 + (NT / 32) * sizeof(WarpWork);
     cudaError_t e = cudaFuncSetAttribute(k_advance<NT, MINB, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e != cudaSuccess) return e;
@@ -569,15 +663,14 @@ cudaError_t launch_advance_stats(const DScene& Sl, const TraceArgs& A, const Wav
 }
 
 // `budget`: dynamic shared memory a block may use; what the warps' work areas
-// leave of it holds nodes.  The FP64 node test reads its nodes from global
-// memory.  The statistics-free instance unless the call collects statistics or
+// leave of it holds node records.  The statistics-free instance unless the call collects statistics or
 // a per-ray work profile.
 template <int NT, int MINB>
 cudaError_t launch_advance_shape(const DScene& S, const TraceArgs& A, const WaveArgs& W, int sm_count, int budget,
                                  cudaStream_t stream) {
     DScene Sl = S;
-    const int room = (budget - (NT / 32) * static_cast<int>(sizeof(WarpWork)) - 16) / 40;
-    Sl.smem_nodes = W.node_f32 ? std::min(S.n_nodes, std::max(room, 0)) : 0;
+    const int room = (budget - (NT / 32) * static_cast<int>(sizeof(WarpWork))) / 64;
+    Sl.smem_pairs = std::min(S.n_pairs, std::max(room, 0));
     if (A.stats || A.ray_work) return launch_advance_stats<NT, MINB, true>(Sl, A, W, sm_count, stream);
     return launch_advance_stats<NT, MINB, false>(Sl, A, W, sm_count, stream);
 }

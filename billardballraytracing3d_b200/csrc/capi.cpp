@@ -39,6 +39,10 @@
 namespace bbrt {
 cudaError_t launch_rays(const DScene& S, const TraceArgs& A, const WaveArgs& W, const NewtonRequest* reqs, const int* rays,
                         long long n, int sm_count, cudaStream_t stream);
+cudaError_t launch_round(const DScene& S, const TraceArgs& A, const WaveArgs& W, const RoundControl& R, int sm_count,
+                         cudaStream_t stream);
+size_t split_workspace_bytes(long long n);
+void split_layout(void* ws, long long n, WaveArgs& W, NewtonRequest*& req_a, NewtonRequest*& req_b);
 size_t wave_workspace_bytes(long long n);
 void wave_layout(void* ws, long long n, WaveArgs& W, NewtonRequest*& req_a, NewtonRequest*& req_b);
 cudaError_t launch_advance(const DScene& S, const TraceArgs& A, const WaveArgs& W, int sm_count, int shape,
@@ -177,6 +181,8 @@ struct bbrt_scene {
     bbrt::DScene dev;
     bool uploaded = false;
     bool device_ready = false;      // device, stream and events chosen
+    bool has_triangles = false;
+    bool small_leaves = false;      // no leaf has more slots than a split round takes
     bool tables_uploaded = false;   // patch node / field tables on the device
     bool setup_on_device = false;   // coarse grids, cells and cull boxes computed on (and kept only on) the GPU
     int device = 0;
@@ -493,7 +499,7 @@ int upload_node_tables(bbrt_scene* s, const std::vector<double>& nbox, const std
 int build_leaf_tables(bbrt_scene* s, const std::vector<double>& nbox, const std::vector<int>& nlink,
                       const std::vector<int>& roots) {
     bbrt::DScene& D = s->dev;
-    constexpr int kCutLeaves = 32, kMaxDepth = 60;
+    constexpr int kCutLeaves = 32, kMaxDepth = 30;   // (median splits: at most 25)
     const size_t n_slots = s->host.leaf_objects.size(), nn = nlink.size() / 4;
     std::vector<int> leaf_of(nn, -1), below(nn, 0), leaves, cuts, m_cut{ 0 }, cut_first;
     bool shallow = true;
@@ -545,10 +551,21 @@ int build_leaf_tables(bbrt_scene* s, const std::vector<double>& nbox, const std:
             }
         }
     }
+    std::vector<int> pair_of(nn, -1), pair_node, m_ref;
+    for (size_t k = 0; k < nn; ++k)
+        if (nlink[4 * k + 1] >= 0) {
+            pair_of[k] = static_cast<int>(pair_node.size());
+            pair_node.push_back(static_cast<int>(k));
+        }
+    auto ref = [&](int k) { return pair_of[k] >= 0 ? pair_of[k] : ~leaf_of[k]; };
+    for (int root : roots) m_ref.push_back(nn ? ref(root) : 0);
+    const size_t np = pair_node.size();
     auto pad = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
     const size_t at_rec = 0, at_node = at_rec + pad(32 * n_slots), at_box = at_node + pad(32 * nl),
                  at_rank = at_box + pad(48 * nl), at_cut = at_rank + pad(32 * nl), at_cbox = at_cut + pad(32 * ncut),
-                 at_m = at_cbox + pad(48 * ncut), total = at_m + pad(sizeof(int) * m_cut.size());
+                 at_m = at_cbox + pad(48 * ncut), at_pair = at_m + pad(sizeof(int) * m_cut.size()),
+                 at_pnode = at_pair + pad(64 * np), at_ref = at_pnode + pad(sizeof(int) * np),
+                 total = at_ref + pad(sizeof(int) * m_ref.size());
     std::vector<char> blob(total, 0);
     auto record = [&](size_t at, int node, int a, int b) {   // FP32 box and two ints
         float f[6];
@@ -568,6 +585,17 @@ int build_leaf_tables(bbrt_scene* s, const std::vector<double>& nbox, const std:
     }
     if (nl) std::memcpy(&blob[at_rank], rank.data(), 32 * nl);
     std::memcpy(&blob[at_m], m_cut.data(), sizeof(int) * m_cut.size());
+    for (size_t r = 0; r < np; ++r) {
+        const int* l = &nlink[4 * static_cast<size_t>(pair_node[r])];
+        if (l[1] != l[0] + 1) return fail(BBRT_ERR_STATE, "bbrt_scene_upload: siblings are not adjacent");
+        float f[12];
+        for (int k = 0; k < 12; ++k) f[k] = static_cast<float>(nbox[6 * static_cast<size_t>(l[0]) + k]);
+        const int v[4] = { l[0], ref(l[0]), ref(l[1]), l[3] };
+        std::memcpy(&blob[at_pair + 64 * r], f, sizeof f);
+        std::memcpy(&blob[at_pair + 64 * r + 48], v, sizeof v);
+    }
+    if (np) std::memcpy(&blob[at_pnode], pair_node.data(), sizeof(int) * np);
+    std::memcpy(&blob[at_ref], m_ref.data(), sizeof(int) * m_ref.size());
     char* d = nullptr;
     int rc = s->alloc(total, d);
     if (rc) return rc;
@@ -581,7 +609,15 @@ int build_leaf_tables(bbrt_scene* s, const std::vector<double>& nbox, const std:
     D.cut_rec = reinterpret_cast<const float4*>(d + at_cut);
     D.cut_box = reinterpret_cast<const double*>(d + at_cbox);
     D.m_cut = reinterpret_cast<const int*>(d + at_m);
+    D.n_pairs = static_cast<int>(np);
+    D.pair_rec = reinterpret_cast<const float4*>(d + at_pair);
+    D.pair_node = reinterpret_cast<const int*>(d + at_pnode);
+    D.m_ref = reinterpret_cast<const int*>(d + at_ref);
     D.leaf_lists = D.node_f32_ok && shallow ? 1 : 0;
+    s->has_triangles = std::any_of(s->host.kind.begin(), s->host.kind.end(), [](int k) { return k != BBRT_OBJ_PATCH; });
+    s->small_leaves = true;
+    for (size_t l = 0; l < nl; ++l)
+        s->small_leaves = s->small_leaves && nlink[4 * static_cast<size_t>(leaves[l]) + 2] <= bbrt::kSplitLeafSlots;
     return BBRT_OK;
 }
 
@@ -637,9 +673,6 @@ int ensure_uploaded(bbrt_scene* s) {
     // the traversal stack keeps a node index in 24 bits
     if (nn >= (static_cast<size_t>(1) << 24))
         return fail(BBRT_ERR_UNSUPPORTED, "bbrt_scene_upload: more than 16,777,215 BVH nodes");
-    // up to 3400 nodes (64 bytes each, 217 KB) in shared memory; launch shapes
-    // with several blocks per SM stage fewer
-    D.smem_nodes = static_cast<int>(std::min<size_t>(nn, 3400));
     for (int q = 0; q < H.n_patches; ++q) D.max_nodes = std::max(D.max_nodes, std::max(H.p_imax[q], H.p_jmax[q]));
     int rc;
     if ((rc = upload_node_tables(s, nbox, nlink))) return rc;
@@ -1067,6 +1100,17 @@ bool sort_round_requests(const bbrt_scene* s) {
     return tuning().sort_requests && s->host.n_objects >= 1 && s->host.n_objects <= bbrt::request_sort_max_objects();
 }
 
+// Whether a wavefront runs split rounds (k_walk and k_stage1 of rounds.cu) or
+// k_advance rounds.  Split ones need the leaf lists, leaves of few slots and
+// culling; sample recording needs every patch of a visited leaf, in visiting
+// order; and the network knows no triangles.  Same box, split against
+// k_advance: see k_stage1.
+bool split_rounds(const bbrt_scene* s, const bbrt::TraceArgs& A) {
+    const bool learned = s->host.cfg.guess == BBRT_GUESS_LEARNED && s->guess.trained;
+    return s->dev.leaf_lists && s->small_leaves && s->host.cfg.cull && tuning().node_f32 && !A.samples &&
+           !(learned && s->has_triangles);
+}
+
 // Round 0's processing order (s->order): rays bucketed by where they enter
 // the scene's sphere; in a scene set, each member's rays among themselves
 // in its own range, so that warps keep to one member's tree.
@@ -1141,7 +1185,9 @@ int build_wave_graph(bbrt_scene* s, const bbrt::TraceArgs& A, const bbrt_tuning&
     const long long n = A.n;
     bbrt::WaveArgs W;
     bbrt::NewtonRequest *req_a = nullptr, *req_b = nullptr;
-    bbrt::wave_layout(s->wave.p, n, W, req_a, req_b);
+    const bool split = split_rounds(s, A);
+    if (split) bbrt::split_layout(s->wave.p, n, W, req_a, req_b);
+    else bbrt::wave_layout(s->wave.p, n, W, req_a, req_b);
     unsigned int* c = static_cast<unsigned int*>(s->wave_ctr.p);
     W.counters = c;
     W.resume_queries = tuning().resume_queries;
@@ -1174,8 +1220,14 @@ int build_wave_graph(bbrt_scene* s, const bbrt::TraceArgs& A, const bbrt_tuning&
     Wo.count_dev = c + 1;                  // rays that overflowed the resolved list
     const bbrt::MlpNet net = learned ? guess_net(s) : bbrt::MlpNet();
     auto round = [&](cudaStream_t q, const bbrt::WaveArgs& Wa, cudaGraphConditionalHandle loop) -> cudaError_t {
-        cudaError_t e = bbrt::launch_advance(s->dev, A, Wa, s->sm_count, T.advance_shape, q);
-        if (e == cudaSuccess) e = bbrt::launch_wave_decide(c, T.wave_tail, max_rounds, loop, q);
+        bbrt::RoundControl R;
+        R.on = 1;
+        R.wave_tail = T.wave_tail;
+        R.max_rounds = max_rounds;
+        R.loop = loop;
+        cudaError_t e = split ? bbrt::launch_round(s->dev, A, Wa, R, s->sm_count, q)
+                              : bbrt::launch_advance(s->dev, A, Wa, s->sm_count, T.advance_shape, q);
+        if (e == cudaSuccess && !split) e = bbrt::launch_wave_decide(c, T.wave_tail, max_rounds, loop, q);
         if (e == cudaSuccess && sort)
             e = bbrt::sort_requests(req_a, n, c + bbrt::kWcNext, s->host.n_objects, tuning().sort_side,
                                     s->dev.coarse_n - 1, s->order_ws.p, req_b, q);
@@ -1235,7 +1287,7 @@ int build_wave_graph(bbrt_scene* s, const bbrt::TraceArgs& A, const bbrt_tuning&
     }
     out.graph = g;
     out.exec = x;
-    // advance, decide, [4 sort kernels], [infer], Newton
+    // advance, decide (or walk, stage 1), [4 sort kernels], [infer], Newton
     const long long per_round = 3 + (learned ? 1 : 0) + (sort ? 4 : 0);
     out.launches_round = per_round;
     out.launches_fixed = (T.order_rays ? 4 : 0) + per_round + 2;
@@ -1277,7 +1329,7 @@ int launch_wave_graph(bbrt_scene* s, const bbrt::TraceArgs& A, const bbrt_tuning
                          static_cast<long long>(tuning().node_f32), static_cast<long long>(tuning().adapt_lanes),
                          tuning().newton_group_max, max_rounds,
                          static_cast<long long>(sort_round_requests(s)), watchdog_cycles(T), mma_wait_cycles(T),
-                         static_cast<long long>(A.off_patch_miss) })
+                         static_cast<long long>(A.off_patch_miss), static_cast<long long>(split_rounds(s, A)) })
         k.put(x);
     k.put(s->guess.min_logit);
     k.put(s->guess.t_window);
@@ -1321,7 +1373,7 @@ struct WaveRun {
     bbrt::WaveArgs W;
     bbrt::NewtonRequest *req_a = nullptr, *req_b = nullptr;
     long long round = 0, max_rounds = 0, overflowed = 0;
-    bool done = false;
+    bool done = false, split = false;
     GraphLaunch graph;   // graph-launched: check_wave_graph() after completion
 
     int begin(bbrt_scene* s_, const bbrt::TraceArgs& A_, cudaStream_t st_) {
@@ -1331,7 +1383,8 @@ struct WaveRun {
         const long long n = A.n;
         T = scene_tuning(s);
         log_rounds = tuning().log_rounds;
-        BBRT_CUDA(s->wave.ensure(bbrt::wave_workspace_bytes(n)));
+        split = split_rounds(s, A);
+        BBRT_CUDA(s->wave.ensure(split ? bbrt::split_workspace_bytes(n) : bbrt::wave_workspace_bytes(n)));
         BBRT_CUDA(s->wave_ctr.ensure(bbrt::kWaveCounters * sizeof(unsigned int)));
         if (!s->wave_ctr_host)
             BBRT_CUDA(cudaMallocHost(&s->wave_ctr_host, bbrt::kWaveCounters * sizeof(unsigned int)));
@@ -1339,7 +1392,8 @@ struct WaveRun {
             done = true;
             return launch_wave_graph(s, A, T, st, graph);
         }
-        bbrt::wave_layout(s->wave.p, n, W, req_a, req_b);
+        if (split) bbrt::split_layout(s->wave.p, n, W, req_a, req_b);
+        else bbrt::wave_layout(s->wave.p, n, W, req_a, req_b);
         if (sort_round_requests(s)) BBRT_CUDA(s->order_ws.ensure(bbrt::ray_order_workspace_bytes(n)));
         W.counters = static_cast<unsigned int*>(s->wave_ctr.p);
         W.resume_queries = tuning().resume_queries;
@@ -1367,8 +1421,11 @@ struct WaveRun {
         if (log_rounds) BBRT_CUDA(cudaEventRecord(s->ev[2], st));
         BBRT_CUDA(cudaMemsetAsync(W.counters, 0, sizeof(unsigned int), st));
         BBRT_CUDA(cudaMemsetAsync(W.counters + 2, 0, sizeof(unsigned int), st));
-        BBRT_CUDA(timed(s, K_ADVANCE, st,
-                        [&] { return bbrt::launch_advance(s->dev, A, W, s->sm_count, T.advance_shape, st); }));
+        BBRT_CUDA(timed(s, K_ADVANCE, st, [&] {
+            return split ? bbrt::launch_round(s->dev, A, W, bbrt::RoundControl(), s->sm_count, st)
+                         : bbrt::launch_advance(s->dev, A, W, s->sm_count, T.advance_shape, st);
+        }));
+        if (split) ++s->launches;   // two kernels
         ++s->rounds;
         if (log_rounds) BBRT_CUDA(cudaEventRecord(s->ev[3], st));
         BBRT_CUDA(cudaMemcpyAsync(s->wave_ctr_host, W.counters, 4 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
@@ -3081,7 +3138,6 @@ int build_scene_set(const std::vector<bbrt_scene*>& mem, bbrt_scene_set* set) {
     D.sag_factor = H0.cfg.sagitta_clearance_factor;
     D.backface_tol = H0.cfg.backface_tol;
     D.precision = mem[0]->dev.precision;
-    D.smem_nodes = static_cast<int>(std::min<size_t>(NN, 3400));
     D.block_cells = cull_block_cells;
     D.n_blocks_side = cull_blocks;
     D.cull_enabled = 0;   // per member (m_param); a ray without a member never occurs in a set

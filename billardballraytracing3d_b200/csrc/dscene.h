@@ -55,7 +55,17 @@ struct DScene {
     const float4* cut_rec = nullptr;
     const double* cut_box = nullptr;
     const int* m_cut = nullptr;
-    int smem_nodes = 0;                    // nodes [0, smem_nodes) staged in shared memory (k_advance)
+    // The tree's internal nodes for k_advance, breadth-first: a record holds
+    // both children, as four float4: their FP32 boxes (left, then right: 12
+    // floats), then as int bits the left child's node index (the right one's
+    // follows it), the children's references and the split axis.  A reference
+    // is a record index, or ~leaf for a leaf (in leaf_node's order).
+    // pair_node[r]: node index of record r; m_ref: reference of each tree's root.
+    int n_pairs = 0;
+    const float4* pair_rec = nullptr;
+    const int* pair_node = nullptr;
+    const int* m_ref = nullptr;
+    int smem_pairs = 0;                    // records [0, smem_pairs) staged in shared memory
     // FP32 copies of the node boxes (nearest rounding) for the FP32 node
     // test, and per axis a bound on |coordinate| over every node box (FP32,
     // rounded up, at least 2^-60); node_f32_ok = 0 when a bound exceeds 2^40
@@ -186,6 +196,23 @@ struct NewtonRequest {
 constexpr int kResolved = 4;
 constexpr int kResData = 11;
 
+// Split rounds (rounds.cu): leaves a ray's query may list, slots a leaf may
+// have, stage-1 hits and Newton results kept per ray.
+constexpr int kSplitLeaves = 32, kSplitLeafSlots = 4, kSplitHits = 8, kSplitResults = 2;
+
+// One stage-1 hit of a ray's query, in visiting order.
+struct SplitHit {
+    double t;
+    int obj, leaf, key, pad;
+};
+
+// Round control of a graph-launched split round (its last k_stage1 block).
+struct RoundControl {
+    int on = 0;
+    long long wave_tail = 0, max_rounds = 0;
+    cudaGraphConditionalHandle loop = 0;
+};
+
 // Workspace of the wavefront trace (advance / Newton rounds).
 struct WaveArgs {
     double* o = nullptr;       // [n][3] ray state between rounds
@@ -194,7 +221,17 @@ struct WaveArgs {
     int* nres = nullptr;
     int* res_obj = nullptr;    // [n][kResolved]
     int* res_err = nullptr;    // [n][kResolved]
-    double* res_data = nullptr;  // [n][kResolved][kResData]
+    double* res_data = nullptr;  // [n][results][kResData]
+    int results = kResolved;     // results per ray (kSplitResults in split rounds); a request's entry is
+                                 // its result's slot, in split rounds with the hit's place << 1
+    // Split rounds: a query's leaves in visiting order, its stage-1 hits, the
+    // best result so far (hit << 1 | slot, -1 none), the rays that have leaves
+    int* leaves = nullptr;       // [n][kSplitLeaves]
+    int* n_leaves = nullptr;
+    SplitHit* hits = nullptr;    // [n][kSplitHits]
+    int* n_hits = nullptr;
+    int* best = nullptr;
+    int* listed = nullptr;
     const NewtonRequest* runnable = nullptr;   // previous round's requests (null: round 0, all rays)
     const int* order = nullptr;                // round 0 processing order (null: index order)
     long long n_runnable = 0;
@@ -247,7 +284,9 @@ constexpr int kWcRounds = 6;   // rounds whose requests went to Newton
 constexpr int kWcBound = 7;    // the round bound was reached
 constexpr int kWcTailNext = 8; // next slot of the tail kernel (rays handed out one at a time)
 constexpr int kWcOvfNext = 9;  // next slot of the overflow tail
-constexpr int kWaveCounters = 10;
+constexpr int kWcTicket = 10;  // k_stage1 blocks that are done (the last one decides the round)
+constexpr int kWcGroup = 11;   // next ray of the round's list for k_stage1
+constexpr int kWaveCounters = 12;
 
 constexpr int kQsInt = 5;
 constexpr int kSaveStack = 24;

@@ -63,9 +63,8 @@ struct RayWork {
 };
 
 // node_box_f32 on a record's box.
-__device__ __forceinline__ int rec_box_f32(const float4& a, const float4& b, const CullRay& c, float e, double best_t) {
-    __align__(8) const float box[6] = { a.x, a.y, a.z, a.w, b.x, b.y };
-    return node_box_f32(box, c, e, best_t);
+__device__ __forceinline__ int rec_box_f32(const float4& a, const float4& b, const NodeRay& r) {
+    return node_box_f32(a.x, a.y, a.z, a.w, b.x, b.y, r);
 }
 
 // BVH::intersect by walking the tree with a whole warp (every lane returns the
@@ -343,8 +342,8 @@ __device__ __forceinline__ bool ray_query(const DScene& S, RayWork& w, const V3&
     const int oct = (inv[0] < 0.0 ? 1 : 0) | (inv[1] < 0.0 ? 2 : 0) | (inv[2] < 0.0 ? 4 : 0);
     const bool use_cull = cull_ok(S, member, cull_flag, o, d);
     const CullRay cr = make_cull_ray(S, member, o, d);
-    float e32 = 0.0f;
-    const bool node32 = node_margin(S, cr, e32);
+    NodeRay nr;
+    const bool node32 = make_node_ray(S, cr, nr);
     // ---- leaves whose box the ray meets
     const int c_end = S.m_cut[member < 0 ? 1 : member + 1];
     int n_leaf = 0;
@@ -357,7 +356,7 @@ __device__ __forceinline__ bool ray_query(const DScene& S, RayWork& w, const V3&
             first = __float_as_int(b.z);
             count = __float_as_int(b.w);
             // only a filter: undecided subtrees are looked into
-            pass = node32 ? rec_box_f32(a, b, cr, e32, CUDART_INF) != 0 : ray_box_exact(o, inv, S.cut_box + 6LL * k, CUDART_INF);
+            pass = node32 ? rec_box_f32(a, b, nr) != 0 : ray_box_exact(o, inv, S.cut_box + 6LL * k, CUDART_INF);
         }
         if constexpr (Ctr::kOn) {
             if (lane == 0) ctr.node_tests += min(32, c_end - k0);
@@ -368,7 +367,7 @@ __device__ __forceinline__ bool ray_query(const DScene& S, RayWork& w, const V3&
             bool in = false;
             int dec = 0;
             if (lane < cnt) {
-                dec = node32 ? rec_box_f32(S.leaf_node[2LL * l], S.leaf_node[2LL * l + 1], cr, e32, CUDART_INF) : -1;
+                dec = node32 ? rec_box_f32(S.leaf_node[2LL * l], S.leaf_node[2LL * l + 1], nr) : -1;
                 in = dec < 0 ? ray_box_exact(o, inv, S.leaf_box + 6LL * l, CUDART_INF) : dec != 0;
             }
             const unsigned m = __ballot_sync(kFull, in);

@@ -74,17 +74,22 @@ __device__ __forceinline__ CullRay make_cull_ray(const DScene& S, int m, const V
         const double* p = S.m_param + m * kMemberParams;
         ca = p[2]; ch = p[3]; cb = p[4]; cc = p[5]; cr = p[6]; c0 = p[7]; c1 = p[8]; c2 = p[9];
     }
-    const double cx = o.x - c0, cy = o.y - c1, cz = o.z - c2;
-    const double L = sqrt(cx * cx + cy * cy + cz * cz) + cr;
-    const double on = sqrt(o.x * o.x + o.y * o.y + o.z * o.z);
-    const double delta = ca * (L + ch) + cb * (L + on + cc);
+    // upper bounds in FP32, every step rounded up (two FP64 square roots cost
+    // more than the rest of a query's start)
+    const float cx = __double2float_ru(fabs(o.x - c0)), cy = __double2float_ru(fabs(o.y - c1)),
+                cz = __double2float_ru(fabs(o.z - c2));
+    const float ax = __double2float_ru(fabs(o.x)), ay = __double2float_ru(fabs(o.y)), az = __double2float_ru(fabs(o.z));
+    const float L = __fadd_ru(__fsqrt_ru(__fmaf_ru(cx, cx, __fmaf_ru(cy, cy, __fmul_ru(cz, cz)))), __double2float_ru(cr));
+    const float on = __fsqrt_ru(__fmaf_ru(ax, ax, __fmaf_ru(ay, ay, __fmul_ru(az, az))));
+    const float delta = __fmaf_ru(__double2float_ru(ca), __fadd_ru(L, __double2float_ru(ch)),
+                                  __fmul_ru(__double2float_ru(cb), __fadd_ru(__fadd_ru(L, on), __double2float_ru(cc))));
     c.ox = static_cast<float>(o.x);
     c.oy = static_cast<float>(o.y);
     c.oz = static_cast<float>(o.z);
     c.ix = 1.0f / static_cast<float>(d.x);
     c.iy = 1.0f / static_cast<float>(d.y);
     c.iz = 1.0f / static_cast<float>(d.z);
-    c.delta = __double2float_ru(delta * 1.0001);
+    c.delta = __fmul_ru(delta, 1.0001f);
     return c;
 }
 
@@ -93,10 +98,7 @@ __device__ __forceinline__ CullRay make_cull_ray(const DScene& S, int m, const V
 // always passes (the inflation bounds both roundings); only work is skipped.
 // Boxes are 6 floats on a 24-byte stride from a 16-byte aligned array
 // (checked at upload): read as three 8-byte loads.
-__device__ __forceinline__ bool cull_box(const float* __restrict__ b, const CullRay& c) {
-    const float2 b01 = *reinterpret_cast<const float2*>(b);
-    const float2 b23 = *reinterpret_cast<const float2*>(b + 2);
-    const float2 b45 = *reinterpret_cast<const float2*>(b + 4);
+__device__ __forceinline__ bool cull_box(const float2& b01, const float2& b23, const float2& b45, const CullRay& c) {
     float t1 = (b01.x - c.delta - c.ox) * c.ix, t2 = (b23.y + c.delta - c.ox) * c.ix;
     float tmin = fmaxf(0.0f, fminf(t1, t2)), tmax = fmaxf(t1, t2);
     t1 = (b01.y - c.delta - c.oy) * c.iy; t2 = (b45.x + c.delta - c.oy) * c.iy;
@@ -104,6 +106,11 @@ __device__ __forceinline__ bool cull_box(const float* __restrict__ b, const Cull
     t1 = (b23.x - c.delta - c.oz) * c.iz; t2 = (b45.y + c.delta - c.oz) * c.iz;
     tmin = fmaxf(tmin, fminf(t1, t2)); tmax = fminf(tmax, fmaxf(t1, t2));
     return tmin <= tmax;
+}
+
+__device__ __forceinline__ bool cull_box(const float* __restrict__ b, const CullRay& c) {
+    return cull_box(*reinterpret_cast<const float2*>(b), *reinterpret_cast<const float2*>(b + 2),
+                    *reinterpret_cast<const float2*>(b + 4), c);
 }
 
 // One leaf slot's record (DScene::leaf_rec).
@@ -146,40 +153,52 @@ __device__ __forceinline__ int nth_bit(unsigned m, int n) {
 // axes, tmin = max(lo_a) <= tmax = min(hi_a), tmin <= best_t and tmax >= 0,
 // where lo_a / hi_a are the FP64 slab times fl(fl(b - o) * fl(1/d)) of the
 // near / far face (its early exit and swap give that; every t is finite for
-// finite o and 1/d).  The same times in FP32 from b32 = fl32(b), o32 =
-// fl32(o) and 1/fl32(d) (the cull ray's values), each face
-// fl32(fl32(b32 - o32) * i32), differ from the FP64 ones by at most
-// (5 * 2^-24 + 2 * 2^-53) (|b| + |o|) |1/d| plus underflow terms below 2^-120
-// (roundings of b and o: 1, of d and the division: 2, of the subtraction and
-// the product: 1 each, in units of 2^-24 (|b| + |o|) |1/d|); e
-// (node_margin) bounds that with 2^-21 (B_a + |o32_a|) |i32_a| for the
-// largest axis, B_a bounding every node coordinate on axis a.  So
-// [tmin32 - e, tmin32 + e] holds the FP64 tmin and likewise tmax, and the
-// test decides wherever the interval decides: 1 = passes, 0 = fails, -1 =
-// undecided (run ray_box_exact).  Boxes are 6 floats (min xyz, max xyz) on a
-// 24-byte stride, read as three 8-byte loads.
-__device__ __forceinline__ int node_box_f32(const float* __restrict__ b, const CullRay& c, float e, double best_t) {
-    const float2 b01 = *reinterpret_cast<const float2*>(b);
-    const float2 b23 = *reinterpret_cast<const float2*>(b + 2);
-    const float2 b45 = *reinterpret_cast<const float2*>(b + 4);
-    float t1 = (b01.x - c.ox) * c.ix, t2 = (b23.y - c.ox) * c.ix;
+// finite o and 1/d).  In FP32, with b32 = fl32(b), o32 = fl32(o), i32 =
+// fl32(1 / fl32(d)) and p32 = fl32(-o32 * i32), each face's time is one
+// fused multiply-add, fl32(b32 * i32 + p32).  It differs from the FP64 one by
+// at most (5.01 * 2^-24 + 3 * 2^-53) (|b| + |o|) |1/d| plus underflow terms
+// below 2^-120 (in units of 2^-24 |1/d|: roundings of b 1, of o 1, of d and
+// the division 2 for each of b and o, of p 1, of the sum 1); e (make_node_ray)
+// bounds that with 2^-21 (B_a + |o32_a|) |i32_a| for the largest axis, B_a
+// bounding every node coordinate on axis a.  So the FP64 tmin lies within e of
+// the FP32 one and likewise tmax, and the test decides wherever those intervals
+// decide (directed rounding on the sums): 1 = passes, 0 = fails, -1 =
+// undecided (run ray_box_exact).
+struct NodeRay {
+    float ix, iy, iz, px, py, pz;   // 1/d, -o/d
+    float e, e2;                    // margin, and 2 e rounded up
+    float best_hi, best_lo;         // best_t + e rounded up, best_t - e rounded down
+    __device__ __forceinline__ void set_best(double best_t) {
+        best_hi = __fadd_ru(__double2float_ru(best_t), e);
+        best_lo = __fsub_rd(__double2float_rd(best_t), e);
+    }
+};
+
+__device__ __forceinline__ int node_box_f32(float x0, float y0, float z0, float x1, float y1, float z1, const NodeRay& r) {
+    float t1 = fmaf(x0, r.ix, r.px), t2 = fmaf(x1, r.ix, r.px);
     float tmin = fminf(t1, t2), tmax = fmaxf(t1, t2);
-    t1 = (b01.y - c.oy) * c.iy; t2 = (b45.x - c.oy) * c.iy;
+    t1 = fmaf(y0, r.iy, r.py); t2 = fmaf(y1, r.iy, r.py);
     tmin = fmaxf(tmin, fminf(t1, t2)); tmax = fminf(tmax, fmaxf(t1, t2));
-    t1 = (b23.x - c.oz) * c.iz; t2 = (b45.y - c.oz) * c.iz;
+    t1 = fmaf(z0, r.iz, r.pz); t2 = fmaf(z1, r.iz, r.pz);
     tmin = fmaxf(tmin, fminf(t1, t2)); tmax = fminf(tmax, fmaxf(t1, t2));
-    const float lo_dn = __fsub_rd(tmin, e), lo_up = __fadd_ru(tmin, e);
-    const float hi_dn = __fsub_rd(tmax, e), hi_up = __fadd_ru(tmax, e);
-    if (lo_dn > hi_up || hi_up < 0.0f || static_cast<double>(lo_dn) > best_t) return 0;
-    if (lo_up <= hi_dn && hi_dn >= 0.0f && static_cast<double>(lo_up) <= best_t) return 1;
+    if (tmin > __fadd_ru(tmax, r.e2) || tmax < -r.e || tmin > r.best_hi) return 0;
+    if (tmin <= __fsub_rd(tmax, r.e2) && tmax >= r.e && tmin <= r.best_lo) return 1;
     return -1;
 }
 
-// The margin e of node_box_f32 for a ray (false: the ray's FP32 values lie
-// outside the range the bound covers, and its node tests stay FP64).  The
-// limits keep every FP32 time below 2^81 and 1/d normal; the 2^-100 floor
-// covers the underflow terms.
-__device__ __forceinline__ bool node_margin(const DScene& S, const CullRay& c, float& e) {
+// A box of 6 floats (min xyz, max xyz), 8-byte aligned: three 8-byte loads.
+__device__ __forceinline__ int node_box_f32(const float* __restrict__ b, const NodeRay& r) {
+    const float2 b01 = *reinterpret_cast<const float2*>(b);
+    const float2 b23 = *reinterpret_cast<const float2*>(b + 2);
+    const float2 b45 = *reinterpret_cast<const float2*>(b + 4);
+    return node_box_f32(b01.x, b01.y, b23.x, b23.y, b45.x, b45.y, r);
+}
+
+// The FP32 node test's ray (false: its values lie outside the range the bound
+// covers, and its node tests stay FP64).  The limits keep every FP32 time below
+// 2^81 and 1/d normal; the 2^-100 floor covers the underflow terms.  best_t is
+// infinite.
+__device__ __forceinline__ bool make_node_ray(const DScene& S, const CullRay& c, NodeRay& r) {
     const float o[3] = { c.ox, c.oy, c.oz }, iv[3] = { c.ix, c.iy, c.iz };
     float m = 0x1p-100f;
     bool ok = S.node_f32_ok != 0;
@@ -189,7 +208,11 @@ __device__ __forceinline__ bool node_margin(const DScene& S, const CullRay& c, f
         ok = ok && ai >= 0x1p-40f && ai <= 0x1p40f && ao <= 0x1p40f;
         m = fmaxf(m, __fmul_ru(__fadd_ru(S.node_bound[a], ao), ai) * 0x1p-21f);
     }
-    e = m;
+    r.ix = c.ix; r.iy = c.iy; r.iz = c.iz;
+    r.px = -c.ox * c.ix; r.py = -c.oy * c.iy; r.pz = -c.oz * c.iz;
+    r.e = m;
+    r.e2 = 2.0f * m;
+    r.best_hi = r.best_lo = CUDART_INF_F;
     return ok;
 }
 
@@ -606,19 +629,8 @@ __device__ __forceinline__ RayCtx load_ray(const TraceArgs& A, const WaveArgs& W
     r.status = -1;
     r.err_obj = -1;
     r.ev0 = r.ev1 = 0.0;
-    nres = W.nres[i];
+    nres = W.nres ? W.nres[i] : 0;
     return r;
-}
-
-// Warp-aggregated append: returns this lane's slot (or -1 when !want).
-__device__ __forceinline__ long long warp_append(unsigned int* counter, bool want) {
-    const unsigned mask = __ballot_sync(0xffffffffu, want);
-    const int lane = threadIdx.x & 31;
-    unsigned int base = 0;
-    if (lane == 0 && mask) base = atomicAdd(counter, static_cast<unsigned int>(__popc(mask)));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (!want) return -1;
-    return static_cast<long long>(base) + __popc(mask & ((1u << lane) - 1u));
 }
 
 // Appends one training sample (learned guess) when recording is on.

@@ -74,7 +74,9 @@ __device__ __forceinline__ void newton_thread_body(const DScene& S, const TraceA
             }
         }
         const QHit h0 = h;
-        const int ok = newton_mode(S, pidx, o, d, su, sv, st, h, iters, iters32);
+        CountersT<false> dummy;
+        const int ok = S.obj_kind[q.obj] == BBRT_OBJ_PATCH ? newton_mode(S, pidx, o, d, su, sv, st, h, iters, iters32)
+                                                           : triangle_intersect(S, pidx, o, d, h, dummy);
         if (used && !(ok && fabs(h.t - q.t0) <= win)) {
             fallback = 1;
             h = h0;
@@ -91,7 +93,7 @@ __device__ __forceinline__ void newton_thread_body(const DScene& S, const TraceA
         if (A.samples && h.err == 0) record_sample(A, 1, o, d, pidx, h.u, h.v, h.t);
         // a root outside the patch teaches the network a miss near the edge
         if (A.samples && h.err == BBRT_RAY_NEWTON_DOMAIN) record_sample(A, 0, o, d, pidx, 0.0, 0.0, 0.0);
-        const long long e = static_cast<long long>(q.ray) * kResolved + q.entry;
+        const long long e = static_cast<long long>(q.ray) * W.results + (q.entry & (W.results - 1));
         double* rd = W.res_data + e * kResData;
         rd[0] = h.t; rd[1] = h.p.x; rd[2] = h.p.y; rd[3] = h.p.z;
         rd[4] = h.n.x; rd[5] = h.n.y; rd[6] = h.n.z; rd[7] = h.u; rd[8] = h.v; rd[9] = h.ev0; rd[10] = h.ev1;
@@ -143,7 +145,10 @@ __device__ __forceinline__ void newton_grp_body(const DScene& S, const TraceArgs
                 }
             }
         }
-        if (!done) {
+        if (S.obj_kind[q.obj] != BBRT_OBJ_PATCH) {
+            CountersT<false> dummy;
+            triangle_intersect(S, pidx, o, d, h, dummy);
+        } else if (!done) {
             double u0, v0;
             key_to_uv(S, q.key, u0, v0);
             grp_newton_mode(S, pidx, o, d, u0, v0, q.t0, h, iters, iters32, G);
@@ -157,7 +162,7 @@ __device__ __forceinline__ void newton_grp_body(const DScene& S, const TraceArgs
         if (G.g == 0) {
             if (A.samples && h.err == 0) record_sample(A, 1, o, d, pidx, h.u, h.v, h.t);
             if (A.samples && h.err == BBRT_RAY_NEWTON_DOMAIN) record_sample(A, 0, o, d, pidx, 0.0, 0.0, 0.0);
-            const long long e = static_cast<long long>(q.ray) * kResolved + q.entry;
+            const long long e = static_cast<long long>(q.ray) * W.results + (q.entry & (W.results - 1));
             double* rd = W.res_data + e * kResData;
             rd[0] = h.t; rd[1] = h.p.x; rd[2] = h.p.y; rd[3] = h.p.z;
             rd[4] = h.n.x; rd[5] = h.n.y; rd[6] = h.n.z; rd[7] = h.u; rd[8] = h.v; rd[9] = h.ev0; rd[10] = h.ev1;
@@ -516,12 +521,13 @@ __global__ void k_node_check(DScene S, const double* __restrict__ o, const doubl
     const double inv[3] = { 1.0 / dd.x, 1.0 / dd.y, 1.0 / dd.z };
     out[2 * i] = ray_box_exact(oo, inv, boxes + 6 * i, best[i]) ? 1 : 0;
     const CullRay c = make_cull_ray(S, -1, oo, dd);
-    float e = 0.0f;
+    NodeRay nr;
     __align__(8) float b32[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) b32[k] = static_cast<float>(boxes[6 * i + k]);
-    const bool ok = finite3(oo) && finite3(dd) && node_margin(S, c, e);
-    out[2 * i + 1] = ok ? node_box_f32(b32, c, e, best[i]) : -2;
+    const bool ok = finite3(oo) && finite3(dd) && make_node_ray(S, c, nr);
+    nr.set_best(best[i]);
+    out[2 * i + 1] = ok ? node_box_f32(b32, nr) : -2;
 }
 
 cudaError_t launch_node_check(const DScene& S, const double* o, const double* d, const double* best, long long n,
