@@ -174,6 +174,9 @@ struct TraceArgs {
     int off_patch_miss = 0;
     // Scene set: the member scene of every ray ([n]); null for one scene.
     const int* ray_member = nullptr;
+    // Single queries run as a round (rounds.cu, ray_warp.cu): bbrt_hit per ray,
+    // directions as they are, nothing else written; null for a trace.
+    void* query_out = nullptr;
 };
 
 // Network outputs (u, v, t, logit) that place a confident hit well inside

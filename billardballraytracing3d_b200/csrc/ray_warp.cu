@@ -543,6 +543,11 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_rays(DScene S, Trac
             r = load_ray(A, W, i, nres);
         }
         CountersT<STATS> c1;
+        if (A.query_out) {
+            const QHit h = any_query(S, w, r.o, r.d, A.cull, lane, c1, false, r.member);
+            if (lane == 0) write_hit(static_cast<bbrt_hit*>(A.query_out) + i, h);
+            continue;
+        }
         while (r.status < 0) {
             if (r.bounces >= A.max_bounces) { r.status = BBRT_RAY_MAX_BOUNCES; break; }
             if (lane == 0) ++tally.queries;

@@ -43,6 +43,13 @@ __device__ __forceinline__ double* res_of(const WaveArgs& W, int i, int e) {
     return W.res_data + (static_cast<long long>(i) * kSplitResults + e) * kResData;
 }
 
+// Ends a single query: its record is all it writes (finish_ray then has nothing
+// to write).
+__device__ __forceinline__ void end_query(const TraceArgs& A, int i, RayCtx& r, const QHit& h) {
+    write_hit(static_cast<bbrt_hit*>(A.query_out) + i, h);
+    r.status = BBRT_RAY_ESCAPED;
+}
+
 // FP64 node test of ray i from its saved state.
 __device__ __forceinline__ bool saved_box_exact(const WaveArgs& W, int i, const double* box, double best_t) {
     const V3 o = load3(W.o + 3LL * i), d = load3(W.d + 3LL * i);
@@ -126,8 +133,12 @@ __global__ void __launch_bounds__(kWalkThreads, 4) k_walk(DScene S, TraceArgs A,
             CountersT<STATS> cray;
             if (W.runnable == nullptr) {
                 i = W.order ? W.order[j] : static_cast<int>(j);
-                init_outputs(A, i);
-                r = start_ray(A, i);
+                if (A.query_out) {
+                    r = start_query(A, i);
+                } else {
+                    init_outputs(A, i);
+                    r = start_ray(A, i);
+                }
                 if (r.status < 0) {
                     if (A.max_bounces > 0) query = true;
                     else r.status = BBRT_RAY_MAX_BOUNCES;
@@ -185,7 +196,9 @@ __global__ void __launch_bounds__(kWalkThreads, 4) k_walk(DScene S, TraceArgs A,
                         h.ev1 = rd[10];
                     }
                     ++tally.queries;
-                    if (step_ray(S, A, i, r, h)) {
+                    if (A.query_out) {
+                        end_query(A, i, r, h);
+                    } else if (step_ray(S, A, i, r, h)) {
                         if (r.bounces < A.max_bounces) query = true;
                         else r.status = BBRT_RAY_MAX_BOUNCES;
                     }
@@ -211,7 +224,8 @@ __global__ void __launch_bounds__(kWalkThreads, 4) k_walk(DScene S, TraceArgs A,
                         QHit h;
                         h.err = 0;
                         h.obj = -1;
-                        step_ray(S, A, i, r, h);
+                        if (A.query_out) end_query(A, i, r, h);
+                        else step_ray(S, A, i, r, h);
                     } else {
                         W.n_leaves[i] = found;
                         listed = true;
@@ -632,7 +646,8 @@ __global__ void __launch_bounds__(kS1Warps * 32, 6) k_stage1(DScene S, TraceArgs
                 h.err = 0;
                 h.obj = -1;
                 ++tally.queries;
-                step_ray(S, A, i, r, h);
+                if (A.query_out) end_query(A, i, r, h);
+                else step_ray(S, A, i, r, h);
                 finish_ray(A, i, r);
                 tally.bounces += r.bounces;
                 tally.hist[r.status]++;

@@ -466,6 +466,19 @@ __device__ __forceinline__ RayCtx start_ray(const TraceArgs& A, long long i) {
     return r;
 }
 
+// A single query's ray: as given.
+__device__ __forceinline__ RayCtx start_query(const TraceArgs& A, long long i) {
+    RayCtx r;
+    r.o = load3(A.origins + 3 * i);
+    r.d = load3(A.dirs + 3 * i);
+    r.member = -1;
+    r.bounces = 0;
+    r.status = -1;
+    r.err_obj = -1;
+    r.ev0 = r.ev1 = 0.0;
+    return r;
+}
+
 // The last recorded point of a ray, kept in the caller's array from bounce to
 // bounce rather than in the ray's state.
 __device__ __forceinline__ void put_end(const TraceArgs& A, long long i, const V3& p) {
