@@ -61,6 +61,7 @@ cudaError_t ray_order(const double* o, const double* d, long long n, const doubl
                       void* ws, int* order, cudaStream_t stream, bool entry, long long base);
 cudaError_t launch_query(const DScene& S, const QueryArgs& Q, cudaStream_t stream);
 cudaError_t launch_query_warp(const DScene& S, const QueryArgs& Q, int sm_count, cudaStream_t stream);
+cudaError_t launch_quad_boxes(const DScene& S, int n_patches, float* out, cudaStream_t st);
 cudaError_t launch_leaf_records(const DScene& S, int n_slots, float4* out, cudaStream_t st);
 cudaError_t noalloc_prepare();
 cudaError_t launch_trace_noalloc(const DScene& S, TraceArgs A, bool count_hits, long long* hit_counts_out,
@@ -567,8 +568,13 @@ int build_leaf_tables(bbrt_scene* s, const std::vector<double>& nbox, const std:
                  at_rank = at_box + pad(48 * nl), at_cut = at_rank + pad(32 * nl), at_cbox = at_cut + pad(32 * ncut),
                  at_m = at_cbox + pad(48 * ncut), at_pair = at_m + pad(sizeof(int) * m_cut.size()),
                  at_pnode = at_pair + pad(64 * np), at_ref = at_pnode + pad(sizeof(int) * np),
-                 total = at_ref + pad(sizeof(int) * m_ref.size());
-    std::vector<char> blob(total, 0);
+                 hosted = at_ref + pad(sizeof(int) * m_ref.size());
+    // patch count (a set's merged host scene has only the node counts) and the
+    // quadtree boxes where the grid fits them
+    const size_t n_patches = s->host.p_imax.size();
+    const bool quads = D.c_cell_box && D.n_blocks_side > 0 && D.coarse_n >= 2 && D.coarse_n <= 17;
+    const size_t at_quad = hosted, total = at_quad + (quads ? pad(24 * bbrt::kQuadNodes * n_patches) : 0);
+    std::vector<char> blob(hosted, 0);
     auto record = [&](size_t at, int node, int a, int b) {   // FP32 box and two ints
         float f[6];
         for (int k = 0; k < 6; ++k) f[k] = static_cast<float>(nbox[6 * static_cast<size_t>(node) + k]);
@@ -601,7 +607,12 @@ int build_leaf_tables(bbrt_scene* s, const std::vector<double>& nbox, const std:
     char* d = nullptr;
     int rc = s->alloc(total, d);
     if (rc) return rc;
-    BBRT_CUDA(cudaMemcpyAsync(d, blob.data(), total, cudaMemcpyHostToDevice, s->stream));
+    BBRT_CUDA(cudaMemcpyAsync(d, blob.data(), hosted, cudaMemcpyHostToDevice, s->stream));
+    if (quads) {
+        float* q = reinterpret_cast<float*>(d + at_quad);
+        BBRT_CUDA(bbrt::launch_quad_boxes(D, static_cast<int>(n_patches), q, s->stream));
+        D.quad_box = q;
+    }
     BBRT_CUDA(bbrt::launch_leaf_records(D, static_cast<int>(n_slots), reinterpret_cast<float4*>(d + at_rec), s->stream));
     BBRT_CUDA(cudaStreamSynchronize(s->stream));
     D.leaf_rec = reinterpret_cast<const float4*>(d + at_rec);

@@ -106,6 +106,12 @@ struct DScene {
     double cull_center[3] = { 0.0, 0.0, 0.0 };
     double cull_radius = 0.0;
 
+    // Quadtree of a patch's cull boxes for k_stage1 (grids of at most 16 x 16
+    // cells): kQuadNodes boxes a patch, 2 x 2, 4 x 4, 8 x 8 and 16 x 16 of them,
+    // each level in Morton order (a node's four children side by side); a node
+    // without cells has min > max.  Null for larger grids.
+    const float* quad_box = nullptr;       // [n_patches][kQuadNodes][6]
+
     // triangles
     const double* tri = nullptr;           // [n_tri][9]
 
@@ -119,6 +125,7 @@ struct DScene {
     const double* m_param = nullptr;
 };
 
+constexpr int kQuadNodes = 4 + 16 + 64 + 256;
 // Per-member values of a scene set: scene diagonal, cull on (1) / off (0),
 // cull_a, cull_h, cull_b, cull_coord, cull_radius, cull_center xyz.
 constexpr int kMemberParams = 10;

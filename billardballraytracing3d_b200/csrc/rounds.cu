@@ -271,164 +271,214 @@ __global__ void __launch_bounds__(kWalkThreads, 4) k_walk(DScene S, TraceArgs A,
 
 constexpr int kRays = 16;           // rays of a warp
 constexpr int kS1Warps = 4;         // warps per block
-constexpr int kMaxCand = 32 * kSplitLeafSlots + 32;
-constexpr int kBlockUnroll = 2, kCellUnroll = 1;   // box loads in flight per lane (4 and 2: more spills, 1 % slower)
-constexpr int kBlkSmall = 512;      // blocks of a batch of 32 patches of 16 each
-constexpr int kBlkCap = kBlkSmall / 2;   // other grids: 4 bytes an entry, tested when full
-constexpr int kCellCap = 128;
+constexpr int kLeafLanes = 32;      // leaves expanded at a time
+constexpr int kMaxCand = kLeafLanes * kSplitLeafSlots;
+constexpr int kQueue = 80;          // nodes of a quadtree level that wait (at most 15 and 64 new ones)
+constexpr int kBlkCap = 128, kCellCap = 64;   // larger grids: blocks and cells that wait
+
+// A ray's cull test as fused multiply-adds: slab times fma(b, i, p) of the two
+// faces of an axis, inflated, with p = -(o + delta) i for the min face and
+// (delta - o) i for the max face.  Rounding: o, o + delta and the product in p
+// 3 units of 2^-24 (|o| + delta) |i|, 1/d 2 of (|b| + |o| + delta) |i|, the sum
+// 1: 6 (|b| + |o| + delta), as a distance, of the 32 that delta holds for the
+// slab test (cull_constants).  |i| is kept to 1e18, so that an axis the ray does
+// not move along decides by where the origin is; a time of at most t moves it
+// t * 1e-18 there.
+struct __align__(16) CullFma {
+    float ix, iy, iz, nx, ny, nz, xx, xy, xz, pad[3];
+};
+
+// false: a value beyond the range the test is sound in (the ray then goes to the
+// overflow list).
+__device__ __forceinline__ bool make_cull_fma(const CullRay& c, CullFma& f) {
+    f.ix = fminf(fmaxf(c.ix, -1e18f), 1e18f);
+    f.iy = fminf(fmaxf(c.iy, -1e18f), 1e18f);
+    f.iz = fminf(fmaxf(c.iz, -1e18f), 1e18f);
+    f.nx = -(c.ox + c.delta) * f.ix; f.xx = (c.delta - c.ox) * f.ix;
+    f.ny = -(c.oy + c.delta) * f.iy; f.xy = (c.delta - c.oy) * f.iy;
+    f.nz = -(c.oz + c.delta) * f.iz; f.xz = (c.delta - c.oz) * f.iz;
+    const float m = fmaxf(fmaxf(fmaxf(fabsf(f.nx), fabsf(f.xx)), fmaxf(fabsf(f.ny), fabsf(f.xy))),
+                          fmaxf(fabsf(f.nz), fabsf(f.xz)));
+    return m <= 1e37f;
+}
+
+__device__ __forceinline__ bool cull_fma(float x0, float y0, float z0, float x1, float y1, float z1, const CullFma& f) {
+    float t1 = fmaf(x0, f.ix, f.nx), t2 = fmaf(x1, f.ix, f.xx);
+    float tmin = fminf(t1, t2), tmax = fmaxf(t1, t2);
+    t1 = fmaf(y0, f.iy, f.ny); t2 = fmaf(y1, f.iy, f.xy);
+    tmin = fmaxf(tmin, fminf(t1, t2)); tmax = fminf(tmax, fmaxf(t1, t2));
+    t1 = fmaf(z0, f.iz, f.nz); t2 = fmaf(z1, f.iz, f.xz);
+    tmin = fmaxf(fmaxf(tmin, 0.0f), fminf(t1, t2)); tmax = fminf(tmax, fmaxf(t1, t2));
+    return tmin <= tmax;
+}
 
 // One warp's shared memory.
 struct __align__(16) S1Work {
-    float4 cr_a[kRays], cr_b[kRays];           // cull rays: origin, inflation; 1 / direction
+    CullFma cull[kRays];                       // cull tests of the rays
     double od[6][kRays];                       // origins, directions
     int ray[kRays], n_hits[kRays], leaf0[kRays];
     unsigned char leaf_ray[kRays * kSplitLeaves];   // the leaves in (ray, visiting) order: their rays
-    int sub[kMaxCand], slot[kMaxCand];         // candidates in that order: patch or ~triangle, slot
-    unsigned char cand_ray[kMaxCand], cand_pos[kMaxCand];   // ... ray, place of its leaf
-    union {                                    // passing blocks of a batch
-        unsigned short small[kBlkSmall];       // candidate << 8 | row << 4 | column
-        int any[kBlkCap];                      // candidate << 24 | block
-    } blk;
-    int cell[kCellCap];                        // passing cells: candidate of the batch << 24 | cell
+    // candidates in that order: patch or ~triangle, slot, stage-1 winner (key < 0: none), ray, place of its leaf
+    int sub[kMaxCand], slot[kMaxCand], key[kMaxCand];
+    double t[kMaxCand];
+    unsigned char cand_ray[kMaxCand], cand_pos[kMaxCand];
+    int queue[4][kQueue];                      // quadtree nodes, then cells, that passed: candidate << 16 | Morton index
+    int blk[kBlkCap];                          // larger grids: passing blocks, candidate << 24 | block ...
+    int cell[kCellCap];                        // ... and cells
     int cells[kRays], tris[kRays];             // box and triangle tests (statistics)
 };
 
-__device__ __forceinline__ CullRay s1_cull(const S1Work& w, int r) {
-    const float4 a = w.cr_a[r], b = w.cr_b[r];
-    CullRay c;
-    c.ox = a.x; c.oy = a.y; c.oz = a.z; c.delta = a.w;
-    c.ix = b.x; c.iy = b.y; c.iz = b.z;
-    return c;
+// Cell (i, j) of Morton index m (j in the even bits).
+__device__ __forceinline__ void morton_cell(int m, int& i, int& j) {
+    j = (m & 1) | (m >> 1 & 2) | (m >> 2 & 4) | (m >> 3 & 8);
+    m >>= 1;
+    i = (m & 1) | (m >> 1 & 2) | (m >> 2 & 4) | (m >> 3 & 8);
 }
 
-// Triangle tests of the n cells waiting, 32 at a time; a hit goes to the lane of
-// its candidate, which keeps the (t, key) minimum.
-__device__ __forceinline__ void s1_tris(const DScene& S, S1Work& w, int c0, int n_cells, int lane, Stage1& mine) {
-    const int n = S.coarse_n, nc = n - 1, total = 6 * n_cells;
-    for (int p0 = 0; p0 < total; p0 += 32) {
-        const int p = p0 + lane;
-        Stage1 s;
-        int owner = 0;
-        if (p < total) {
-            const int ce = p / 6, e = w.cell[ce], cl = e & 0xFFFFFF, i = cl / nc;
-            owner = e >> 24;
-            const int sub = w.sub[c0 + owner], r = w.cand_ray[c0 + owner];
-            stage1_tri(S.c_xyz + static_cast<long long>(sub) * n * n * 3, S.c_cell + static_cast<long long>(sub) * nc * nc * 4,
-                       n, i, cl - i * nc, p - 6 * ce, v3(w.od[0][r], w.od[1][r], w.od[2][r]),
-                       v3(w.od[3][r], w.od[4][r], w.od[5][r]), s);
+// Triangle tests of up to sixteen cells: a lane takes one of a cell's two
+// triangles at its three offsets (six lanes a cell loaded every corner three
+// times and handed over three times the hits).  A candidate keeps its
+// (t, key) minimum.
+template <class Cell>
+__device__ __forceinline__ void s1_tris(const DScene& S, S1Work& w, int n_cells, int lane, Cell cell_at) {
+    const int n = S.coarse_n, nc = n - 1;
+    Stage1 s;
+    int cand = 0;
+    if (lane < 2 * n_cells) {
+        int i, j;
+        cell_at(lane >> 1, cand, i, j);
+        const int sub = w.sub[cand], r = w.cand_ray[cand];
+        stage1_tri3(S.c_xyz + static_cast<long long>(sub) * n * n * 3, S.c_cell + static_cast<long long>(sub) * nc * nc * 4, n,
+                    i, j, lane & 1, v3(w.od[0][r], w.od[1][r], w.od[2][r]), v3(w.od[3][r], w.od[4][r], w.od[5][r]), s);
+    }
+    for (unsigned hits = __ballot_sync(kFull, s.have); hits; hits &= hits - 1) {
+        if (lane == __ffs(hits) - 1) {
+            Stage1 b;
+            b.key = w.key[cand];
+            b.have = b.key >= 0;
+            b.t = w.t[cand];
+            b.consider(s.t, s.key);
+            w.t[cand] = b.t;
+            w.key[cand] = b.key;
         }
-        for (unsigned hits = __ballot_sync(kFull, s.have); hits; hits &= hits - 1) {
-            const int src = __ffs(hits) - 1;
-            const double t = __shfl_sync(kFull, s.t, src);
-            const int key = __shfl_sync(kFull, s.key, src);
-            const int to = __shfl_sync(kFull, owner, src);
-            if (lane == to) mine.consider(t, key);
-        }
+        __syncwarp();
     }
 }
 
-// Stage 1 of the P <= 32 candidates from c0 on: lane c returns candidate c's
-// winner.  Patches of at most 4 x 4 blocks of 4 x 4 cells: sixteen lanes take a
-// patch's blocks, then a block's cells, several at a time so that their loads
-// are in flight together.
+// Stage 1 of candidates [first, last) by their patches' quadtrees: every step
+// takes eight waiting nodes of one level and tests their four children, a lane
+// each, or sixteen cells' triangles; the deepest level with enough waiting goes
+// first, so the lists stay short and the lanes full (5.3 tests a level and
+// candidate where sixteen blocks and sixteen cells a block were 32).
 template <bool STATS>
-__device__ __forceinline__ Stage1 s1_batch_small(const DScene& S, S1Work& w, int c0, int P, int lane) {
-    const int nc = S.coarse_n - 1, NB = S.n_blocks_side, NB2 = NB * NB;
+__device__ __forceinline__ void s1_quads(const DScene& S, S1Work& w, int first, int last, int lane) {
     const unsigned lt = (1u << lane) - 1u;
-    const int half = lane >> 4, hl = lane & 15;
-    const int hi = hl / NB, hj = hl - hi * NB;
-    Stage1 mine;
-    int n_blk = 0;
-    constexpr int U = kBlockUnroll, V = kCellUnroll;
-    for (int p = 0; p < P; p += 2 * U) {
-        int ray[U];
-        float2 b[U][3];
+    int next = first, n1 = 0, n2 = 0, n3 = 0, n4 = 0;
+    while (true) {
+        int level;
+        if (n4 >= 16) level = 4;
+        else if (n3 >= 16) level = 3;
+        else if (n2 >= 16) level = 2;
+        else if (n1 >= 16) level = 1;
+        else if (next < last) level = 0;
+        else if (n1 > 0) level = 1;
+        else if (n2 > 0) level = 2;
+        else if (n3 > 0) level = 3;
+        else if (n4 > 0) level = 4;
+        else break;
+        if (level == 4) {
+            const int k = min(n4, 16), at = n4 - k;
+            s1_tris(S, w, k, lane, [&](int e, int& cand, int& i, int& j) {
+                const int x = w.queue[3][at + e];
+                cand = x >> 16;
+                morton_cell(x & 0xFFFF, i, j);
+            });
+            n4 = at;
+            continue;
+        }
+        // two nodes' children per lane, their boxes in flight together
+        const int have = level == 0 ? last - next : level == 1 ? n1 : level == 2 ? n2 : n3;
+        const int k = min(have, 16);
+        const int off = level == 0 ? 0 : level == 1 ? 4 : level == 2 ? 20 : 84;
+        int entry[2], ray[2];
+        float2 b[2][3];
 #pragma unroll
-        for (int k = 0; k < U; ++k) {
-            const int c = p + 2 * k + half;
-            ray[k] = -1;
-            if (c < P && hl < NB2) {
-                const int sub = w.sub[c0 + c];
+        for (int u = 0; u < 2; ++u) {
+            const int e = (lane >> 2) + 8 * u;
+            ray[u] = -1;
+            entry[u] = 0;
+            if (e < k) {
+                const int x = level == 0 ? (next + e) << 16 : w.queue[level - 1][have - k + e];
+                const int cand = x >> 16, m = (x & 0xFFFF) * 4 + (lane & 3);
+                entry[u] = cand << 16 | m;
+                const int sub = w.sub[cand];
                 if (sub >= 0) {
-                    ray[k] = w.cand_ray[c0 + c];
-                    const float2* src = reinterpret_cast<const float2*>(S.c_block_box + (static_cast<long long>(sub) * NB2 + hl) * 6);
+                    ray[u] = w.cand_ray[cand];
+                    const float2* q = reinterpret_cast<const float2*>(S.quad_box) + (static_cast<long long>(sub) * kQuadNodes + off + m) * 3;
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) b[k][a] = src[a];
+                    for (int a = 0; a < 3; ++a) b[u][a] = q[a];
                 }
             }
         }
+        int add = 0;
+        int to = level == 0 ? n1 : level == 1 ? n2 : level == 2 ? n3 : n4;
+        __syncwarp();
 #pragma unroll
-        for (int k = 0; k < U; ++k) {
-            if (STATS && ray[k] >= 0) atomicAdd(&w.cells[ray[k]], 1);
-            const bool pass = ray[k] >= 0 && cull_box(b[k][0], b[k][1], b[k][2], s1_cull(w, ray[k]));
-            const unsigned m = __ballot_sync(kFull, pass);
-            if (pass) w.blk.small[n_blk + __popc(m & lt)] = static_cast<unsigned short>((p + 2 * k + half) << 8 | hi << 4 | hj);
-            n_blk += __popc(m);
-        }
-    }
-    __syncwarp();
-    int n_cell = 0;
-    for (int p = 0; p < n_blk; p += 2 * V) {
-        int entry[V];   // candidate << 24 | cell, or -1
-        float2 b[V][3];
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-            const int c = p + 2 * k + half;
-            entry[k] = -1;
-            if (c < n_blk) {
-                const int e = w.blk.small[c], i = ((e >> 4) & 15) * 4 + (hl >> 2), j = (e & 15) * 4 + (hl & 3);
-                if (i < nc && j < nc) {
-                    const int cell = i * nc + j;
-                    entry[k] = (e >> 8) << 24 | cell;
-                    const float2* src = reinterpret_cast<const float2*>(
-                        S.c_cell_box + (static_cast<long long>(w.sub[c0 + (e >> 8)]) * nc * nc + cell) * 6);
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) b[k][a] = src[a];
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-            bool pass = entry[k] >= 0;
+        for (int u = 0; u < 2; ++u) {
+            bool pass = ray[u] >= 0;
             if (pass) {
-                const int r = w.cand_ray[c0 + (entry[k] >> 24)];
-                if (STATS) atomicAdd(&w.cells[r], 1);
-                pass = cull_box(b[k][0], b[k][1], b[k][2], s1_cull(w, r));
-                if (STATS && pass) atomicAdd(&w.tris[r], 6);
+                if (STATS) atomicAdd(&w.cells[ray[u]], 1);
+                pass = b[u][0].x <= b[u][1].y &&
+                       cull_fma(b[u][0].x, b[u][0].y, b[u][1].x, b[u][1].y, b[u][2].x, b[u][2].y, w.cull[ray[u]]);
+                if (STATS && pass && level == 3) atomicAdd(&w.tris[ray[u]], 6);
             }
-            const unsigned m = __ballot_sync(kFull, pass);
-            if (pass) w.cell[n_cell + __popc(m & lt)] = entry[k];
-            n_cell += __popc(m);
+            const unsigned pm = __ballot_sync(kFull, pass);
+            if (pass) w.queue[level][to + add + __popc(pm & lt)] = entry[u];
+            add += __popc(pm);
         }
-        if (n_cell > kCellCap - 32 * V || p + 2 * V >= n_blk) {
-            __syncwarp();
-            s1_tris(S, w, c0, n_cell, lane, mine);
-            __syncwarp();
-            n_cell = 0;
-        }
+        __syncwarp();
+        if (level == 0) { next += k; n1 += add; }
+        else if (level == 1) { n1 -= k; n2 += add; }
+        else if (level == 2) { n2 -= k; n3 += add; }
+        else { n3 -= k; n4 += add; }
     }
-    return mine;
 }
 
-// The same for any grid: blocks and cells flattened over the batch.
+// The same for larger grids: a candidate's blocks, then the cells of the blocks
+// that pass, flattened over the candidates.
 template <bool STATS>
-__device__ __forceinline__ Stage1 s1_batch(const DScene& S, S1Work& w, int c0, int P, int lane) {
+__device__ __forceinline__ void s1_blocks(const DScene& S, S1Work& w, int first, int last, int lane) {
     const int nc = S.coarse_n - 1, B = S.block_cells, B2 = B * B, NB = S.n_blocks_side, NB2 = NB * NB;
     const unsigned lt = (1u << lane) - 1u;
-    Stage1 mine;
     int n_blk = 0, n_cell = 0;
-    const int blocks = P * NB2;
-    for (int b0 = 0; b0 < blocks; b0 += 32) {
-        const int x = b0 + lane, c = x / NB2, b = x - c * NB2;
+    const long long blocks = static_cast<long long>(last - first) * NB2;
+    auto flush = [&] {
+        __syncwarp();
+        for (int at = 0; at < n_cell; at += 16)
+            s1_tris(S, w, min(16, n_cell - at), lane, [&](int e, int& cand, int& i, int& j) {
+                const int x = w.cell[at + e];
+                cand = x >> 24;
+                i = (x & 0xFFFFFF) / nc;
+                j = (x & 0xFFFFFF) - i * nc;
+            });
+        __syncwarp();
+        n_cell = 0;
+    };
+    for (long long b0 = 0; b0 < blocks; b0 += 32) {
+        const long long x = b0 + lane;
+        const int c = first + static_cast<int>(x / NB2), b = static_cast<int>(x % NB2);
         bool pass = x < blocks;
         if (pass) {
-            const int sub = w.sub[c0 + c], r = w.cand_ray[c0 + c];
+            const int sub = w.sub[c], r = w.cand_ray[c];
             pass = sub >= 0;
             if (STATS && pass) atomicAdd(&w.cells[r], 1);
-            if (pass) pass = cull_box(S.c_block_box + (static_cast<long long>(sub) * NB2 + b) * 6, s1_cull(w, r));
+            if (pass) {
+                const float2* q = reinterpret_cast<const float2*>(S.c_block_box + (static_cast<long long>(sub) * NB2 + b) * 6);
+                pass = cull_fma(q[0].x, q[0].y, q[1].x, q[1].y, q[2].x, q[2].y, w.cull[r]);
+            }
         }
         const unsigned m = __ballot_sync(kFull, pass);
-        if (pass) w.blk.any[n_blk + __popc(m & lt)] = c << 24 | b;
+        if (pass) w.blk[n_blk + __popc(m & lt)] = c << 24 | b;
         n_blk += __popc(m);
         if (b0 + 32 < blocks && n_blk <= kBlkCap - 32) continue;
         __syncwarp();
@@ -438,34 +488,29 @@ __device__ __forceinline__ Stage1 s1_batch(const DScene& S, S1Work& w, int c0, i
             bool ok = y < cells;
             int cand = 0, cell = 0;
             if (ok) {
-                const int e = w.blk.any[q], bb = e & 0xFFFFFF, bi = bb / NB, ki = k / B;
+                const int e = w.blk[q], bb = e & 0xFFFFFF, bi = bb / NB, ki = k / B;
                 const int i = bi * B + ki, j = (bb - bi * NB) * B + (k - ki * B);
                 cand = e >> 24;
                 cell = i * nc + j;
                 ok = i < nc && j < nc;
             }
             if (ok) {
-                const int r = w.cand_ray[c0 + cand];
+                const int r = w.cand_ray[cand];
                 if (STATS) atomicAdd(&w.cells[r], 1);
-                ok = cull_box(S.c_cell_box + (static_cast<long long>(w.sub[c0 + cand]) * nc * nc + cell) * 6, s1_cull(w, r));
+                const float2* q2 = reinterpret_cast<const float2*>(S.c_cell_box +
+                                                                   (static_cast<long long>(w.sub[cand]) * nc * nc + cell) * 6);
+                ok = cull_fma(q2[0].x, q2[0].y, q2[1].x, q2[1].y, q2[2].x, q2[2].y, w.cull[r]);
                 if (STATS && ok) atomicAdd(&w.tris[r], 6);
             }
             const unsigned cm = __ballot_sync(kFull, ok);
             if (ok) w.cell[n_cell + __popc(cm & lt)] = cand << 24 | cell;
             n_cell += __popc(cm);
-            if (n_cell > kCellCap - 32) {
-                __syncwarp();
-                s1_tris(S, w, c0, n_cell, lane, mine);
-                __syncwarp();
-                n_cell = 0;
-            }
+            if (n_cell > kCellCap - 32) flush();
         }
         n_blk = 0;
         __syncwarp();
     }
-    s1_tris(S, w, c0, n_cell, lane, mine);
-    __syncwarp();
-    return mine;
+    flush();
 }
 
 // The round control of a graph-launched trace: no requests, or a watchdog stop:
@@ -494,8 +539,8 @@ __device__ void decide_round(unsigned int* c, const RoundControl& R) {
 
 // A warp per up to sixteen rays of W.listed (fewer in a round with fewer rays
 // than the grid's warps can take sixteen of, a power of two that covers it).
-template <bool SMALL, bool STATS>
-__global__ void __launch_bounds__(kS1Warps * 32, 6) k_stage1(DScene S, TraceArgs A, WaveArgs W, RoundControl R) {
+template <bool QUADS, bool STATS>
+__global__ void __launch_bounds__(kS1Warps * 32, 4) k_stage1(DScene S, TraceArgs A, WaveArgs W, RoundControl R) {
     extern __shared__ __align__(16) unsigned char s1_smem[];
     S1Work& w = reinterpret_cast<S1Work*>(s1_smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -516,13 +561,15 @@ __global__ void __launch_bounds__(kS1Warps * 32, 6) k_stage1(DScene S, TraceArgs
         const int rays = static_cast<int>(min(static_cast<long long>(per), n - g));
         // ---- the rays and the list of their leaves
         int i = -1, count = 0;
+        bool over = false;
         if (lane < rays) {
             i = W.listed[g + lane];
             count = W.n_leaves[i];
             const V3 o = load3(W.o + 3LL * i), d = load3(W.d + 3LL * i);
-            const CullRay cr = make_cull_ray(S, A.ray_member ? A.ray_member[i] : -1, o, d);
-            w.cr_a[lane] = make_float4(cr.ox, cr.oy, cr.oz, cr.delta);
-            w.cr_b[lane] = make_float4(cr.ix, cr.iy, cr.iz, 0.0f);
+            CullFma f;
+            over = !make_cull_fma(make_cull_ray(S, A.ray_member ? A.ray_member[i] : -1, o, d), f);
+            w.cull[lane] = f;
+            if (over) count = 0;
             w.od[0][lane] = o.x; w.od[1][lane] = o.y; w.od[2][lane] = o.z;
             w.od[3][lane] = d.x; w.od[4][lane] = d.y; w.od[5][lane] = d.z;
             w.ray[lane] = i;
@@ -540,22 +587,21 @@ __global__ void __launch_bounds__(kS1Warps * 32, 6) k_stage1(DScene S, TraceArgs
         for (int k = 0; k < count; ++k) w.leaf_ray[x - count + k] = static_cast<unsigned char>(lane);
         __syncwarp();
         // ---- a leaf per lane: its patches whose box the ray meets (triangles: all),
-        // then stage 1, 32 of them at a time
-        int n_cand = 0;
-        for (int l0 = 0; l0 < n_leaf; l0 += 32) {
+        // then stage 1 of them
+        for (int l0 = 0; l0 < n_leaf; l0 += kLeafLanes) {
             int r = 0, first = 0, pos = 0;
             unsigned pass = 0;
-            if (l0 + lane < n_leaf) {
+            if (lane < kLeafLanes && l0 + lane < n_leaf) {
                 r = w.leaf_ray[l0 + lane];
                 pos = l0 + lane - w.leaf0[r];
                 const int leaf = W.leaves[static_cast<long long>(w.ray[r]) * kSplitLeaves + pos];
                 const float4 b = S.leaf_node[2LL * leaf + 1];
                 first = __float_as_int(b.z);
                 const int slots = __float_as_int(b.w);
-                const CullRay cr = s1_cull(w, r);
+                const CullFma f = w.cull[r];
                 for (int k = 0; k < slots; ++k) {
                     const LeafRec rec = load_leaf(S, first + k);
-                    if (rec.sub() < 0 || cull_leaf(rec, cr)) pass |= 1u << k;
+                    if (rec.sub() < 0 || cull_fma(rec.a.x, rec.a.y, rec.a.z, rec.a.w, rec.b.x, rec.b.y, f)) pass |= 1u << k;
                     if (STATS && rec.sub() >= 0) {
                         atomicAdd(&w.cells[r], 1);
                         ++ctr.patch_tests;
@@ -568,71 +614,63 @@ __global__ void __launch_bounds__(kS1Warps * 32, 6) k_stage1(DScene S, TraceArgs
                 const int z = __shfl_up_sync(kFull, y, off);
                 if (lane >= off) y += z;
             }
-            int at = n_cand + y - __popc(pass);
+            int at = y - __popc(pass);
             for (unsigned m = pass; m; m &= m - 1, ++at) {
                 const int slot = first + __ffs(m) - 1;
                 w.sub[at] = __float_as_int(S.leaf_rec[2LL * slot + 1].z);
                 w.slot[at] = slot;
+                w.key[at] = -1;
                 w.cand_ray[at] = static_cast<unsigned char>(r);
                 w.cand_pos[at] = static_cast<unsigned char>(pos);
             }
-            n_cand += __shfl_sync(kFull, y, 31);
+            const int n_cand = __shfl_sync(kFull, y, 31);
             __syncwarp();
-            const bool last = l0 + 32 >= n_leaf;
-            int c0 = 0;
-            for (; c0 < n_cand && (last || c0 + 32 <= n_cand); c0 += 32) {
-                const int P = min(32, n_cand - c0);
-                Stage1 s = SMALL ? s1_batch_small<STATS>(S, w, c0, P, lane) : s1_batch<STATS>(S, w, c0, P, lane);
-                if (lane < P && w.sub[c0 + lane] < 0) {
-                    const int q = w.cand_ray[c0 + lane];
-                    QHit h;
-                    CountersT<false> dummy;
-                    s.have = triangle_intersect(S, ~w.sub[c0 + lane], v3(w.od[0][q], w.od[1][q], w.od[2][q]),
-                                                v3(w.od[3][q], w.od[4][q], w.od[5][q]), h, dummy) != 0;
-                    s.t = h.t;
-                    s.key = 0;
-                    ctr.tri_tests += 1;
+            if (QUADS) s1_quads<STATS>(S, w, 0, n_cand, lane);
+            else s1_blocks<STATS>(S, w, 0, n_cand, lane);
+            __syncwarp();
+            // hits in visiting order
+            for (int c0 = 0; c0 < n_cand; c0 += 32) {
+                const int c = c0 + lane;
+                bool hit = c < n_cand;
+                double t = 0.0;
+                int key = 0;
+                if (hit) {
+                    if (w.sub[c] < 0) {
+                        const int q = w.cand_ray[c];
+                        QHit h;
+                        CountersT<false> dummy;
+                        hit = triangle_intersect(S, ~w.sub[c], v3(w.od[0][q], w.od[1][q], w.od[2][q]),
+                                                 v3(w.od[3][q], w.od[4][q], w.od[5][q]), h, dummy) != 0;
+                        t = h.t;
+                        ctr.tri_tests += 1;
+                    } else {
+                        key = w.key[c];
+                        hit = key >= 0;
+                        t = w.t[c];
+                    }
                 }
-                // hits in visiting order
-                const bool hit = lane < P && s.have;
                 const unsigned hm = __ballot_sync(kFull, hit);
                 if (hit) {
-                    const int c = c0 + lane, q = w.cand_ray[c];
+                    const int q = w.cand_ray[c];
                     const unsigned peers = __match_any_sync(hm, q);
                     const int old = w.n_hits[q], place = old + __popc(peers & lt);
                     if (place < kSplitHits) {
                         SplitHit* out = W.hits + static_cast<long long>(w.ray[q]) * kSplitHits + place;
-                        out->t = s.t;
+                        out->t = t;
                         out->obj = __float_as_int(S.leaf_rec[2LL * w.slot[c] + 1].w);
                         out->leaf = W.leaves[static_cast<long long>(w.ray[q]) * kSplitLeaves + w.cand_pos[c]];
-                        out->key = s.key;
+                        out->key = key;
                     }
                     __syncwarp(hm);
                     if (lane == __ffs(peers) - 1) w.n_hits[q] = old + __popc(peers);
                 }
                 __syncwarp();
             }
-            // fewer than 32 left: they go to the front and wait for the next leaves
-            if (!last && c0 > 0) {
-                const int k = c0 + lane;
-                const bool keep = k < n_cand;
-                const int sub = keep ? w.sub[k] : 0, slot = keep ? w.slot[k] : 0;
-                const unsigned char cr = keep ? w.cand_ray[k] : 0, cp = keep ? w.cand_pos[k] : 0;
-                __syncwarp();
-                if (keep) {
-                    w.sub[lane] = sub;
-                    w.slot[lane] = slot;
-                    w.cand_ray[lane] = cr;
-                    w.cand_pos[lane] = cp;
-                }
-                n_cand -= c0;
-                __syncwarp();
-            }
         }
         // ---- each ray's first hit is its Newton request; none: it escapes
-        bool ask = false, over = false;
+        bool ask = false;
         NewtonRequest rq;
-        if (lane < rays) {
+        if (lane < rays && !over) {
             const int hits = w.n_hits[lane];
             if (hits == 0) {
                 RayCtx r;
@@ -702,18 +740,18 @@ __global__ void __launch_bounds__(kS1Warps * 32, 6) k_stage1(DScene S, TraceArgs
     }
 }
 
-template <bool SMALL, bool STATS>
+template <bool QUADS, bool STATS>
 cudaError_t launch_stage1(const DScene& S, const TraceArgs& A, const WaveArgs& W, const RoundControl& R, int sm_count,
                           cudaStream_t stream) {
     constexpr int smem = kS1Warps * sizeof(S1Work);
-    cudaError_t e = cudaFuncSetAttribute(k_stage1<SMALL, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(k_stage1<QUADS, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int per_sm = 0;
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage1<SMALL, STATS>, kS1Warps * 32, smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage1<QUADS, STATS>, kS1Warps * 32, smem);
     if (e != cudaSuccess) return e;
     const long long blocks = std::min<long long>(static_cast<long long>(std::max(per_sm, 1)) * sm_count,
                                                  (W.n_runnable + kS1Warps - 1) / kS1Warps);
-    k_stage1<SMALL, STATS><<<static_cast<unsigned>(blocks), kS1Warps * 32, smem, stream>>>(S, A, W, R);
+    k_stage1<QUADS, STATS><<<static_cast<unsigned>(blocks), kS1Warps * 32, smem, stream>>>(S, A, W, R);
     return cudaGetLastError();
 }
 
@@ -737,11 +775,11 @@ cudaError_t launch_walk(const DScene& S, const TraceArgs& A, const WaveArgs& W, 
 cudaError_t launch_round(const DScene& S, const TraceArgs& A, const WaveArgs& W, const RoundControl& R, int sm_count,
                          cudaStream_t stream) {
     if (W.n_runnable <= 0) return cudaSuccess;
-    const bool stats = A.stats || A.ray_work, small = S.block_cells == 4 && S.n_blocks_side <= 4;
+    const bool stats = A.stats || A.ray_work, quads = S.quad_box != nullptr;
     const cudaError_t e = stats ? launch_walk<true>(S, A, W, sm_count, stream) : launch_walk<false>(S, A, W, sm_count, stream);
     if (e != cudaSuccess) return e;
-    if (stats) return small ? launch_stage1<true, true>(S, A, W, R, sm_count, stream) : launch_stage1<false, true>(S, A, W, R, sm_count, stream);
-    return small ? launch_stage1<true, false>(S, A, W, R, sm_count, stream) : launch_stage1<false, false>(S, A, W, R, sm_count, stream);
+    if (stats) return quads ? launch_stage1<true, true>(S, A, W, R, sm_count, stream) : launch_stage1<false, true>(S, A, W, R, sm_count, stream);
+    return quads ? launch_stage1<true, false>(S, A, W, R, sm_count, stream) : launch_stage1<false, false>(S, A, W, R, sm_count, stream);
 }
 
 size_t split_workspace_bytes(long long n) {

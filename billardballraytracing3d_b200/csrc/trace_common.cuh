@@ -686,6 +686,31 @@ __device__ __forceinline__ void stage1_tri(const double* __restrict__ X, const d
     if (hit) best.consider(t, (i * nc + j) * 6 + step);
 }
 
+// One of the two triangles of cell (i, j) (second: q00, q11, q01) at all three
+// signs, in stage1_tri's order and arithmetic, its corners loaded once.
+__device__ __forceinline__ void stage1_tri3(const double* __restrict__ X, const double* __restrict__ CC, int n, int i,
+                                            int j, bool second, const V3& o, const V3& d, Stage1& best) {
+    const int nc = n - 1;
+    const double* r0 = X + static_cast<long long>(i * n + j) * 3;
+    const double* r1 = r0 + 3 * n;
+    const double* c = CC + static_cast<long long>(i * nc + j) * 4;
+    const double2 c01 = *reinterpret_cast<const double2*>(c);
+    const double2 c23 = *reinterpret_cast<const double2*>(c + 2);
+    const V3 cn = v3(c01.x, c01.y, c23.x);
+    // the triangle's second and third corner: (q10, q11), or (q11, q01)
+    const V3 p0 = load3(r0), p1 = load3(second ? r1 + 3 : r1), p2 = load3(second ? r0 + 3 : r1 + 3);
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k) {
+        const double sg = (k == 0) ? 0.0 : ((k == 1) ? 1.0 : -1.0);
+        const double dd = sg * c23.y;
+        const V3 q0 = v3(p0.x + cn.x * dd, p0.y + cn.y * dd, p0.z + cn.z * dd);
+        const V3 q1 = v3(p1.x + cn.x * dd, p1.y + cn.y * dd, p1.z + cn.z * dd);
+        const V3 q2 = v3(p2.x + cn.x * dd, p2.y + cn.y * dd, p2.z + cn.z * dd);
+        double t;
+        if (mt_exact(o, d, q0, q1, q2, t)) best.consider(t, (i * nc + j) * 6 + 2 * k + (second ? 1 : 0));
+    }
+}
+
 // ---- warp-cooperative stage 1 (used by k_advance and the warp-per-ray kernels) ----
 
 constexpr unsigned kFull = 0xffffffffu;

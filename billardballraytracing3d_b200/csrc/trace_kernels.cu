@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(128) k_newton_grp(DScene S, TraceArgs A, WaveA
 // small one (at most W.newton_group_max requests, and the grid has their
 // lanes), whose time is its slowest solve's latency.  Same results bit for
 // bit either way.
-__global__ void __launch_bounds__(128) k_newton_auto(DScene S, TraceArgs A, WaveArgs W, long long n_req) {
+__global__ void __launch_bounds__(128, 4) k_newton_auto(DScene S, TraceArgs A, WaveArgs W, long long n_req) {
     if (W.count_dev) n_req = *W.count_dev;
     if (n_req <= W.newton_group_max && n_req * kGroup <= static_cast<long long>(gridDim.x) * blockDim.x)
         newton_grp_body(S, A, W, n_req);
@@ -441,6 +441,47 @@ __global__ void k_leaf_records(DScene S, int n_slots, float4* __restrict__ out) 
     }
     out[2LL * k] = make_float4(lo[0], lo[1], lo[2], hi[0]);
     out[2LL * k + 1] = make_float4(hi[1], hi[2], __int_as_float(patch ? sub : ~sub), __int_as_float(obj));
+}
+
+// DScene::quad_box: a block of 256 threads per patch; thread m takes the cell
+// with Morton index m, then the union of four children level by level.
+__global__ void __launch_bounds__(256) k_quad_boxes(DScene S, float* __restrict__ out) {
+    __shared__ float box[256][6];
+    const int nc = S.coarse_n - 1, m = threadIdx.x;
+    const float* cells = S.c_cell_box + 6LL * nc * nc * blockIdx.x;
+    float* q = out + 6LL * kQuadNodes * blockIdx.x;
+    int i = 0, j = 0;
+    for (int b = 0; b < 4; ++b) {
+        j |= (m >> (2 * b) & 1) << b;
+        i |= (m >> (2 * b + 1) & 1) << b;
+    }
+    const bool in = i < nc && j < nc;
+    for (int a = 0; a < 6; ++a) box[m][a] = in ? cells[6 * (i * nc + j) + a] : (a < 3 ? CUDART_INF_F : -CUDART_INF_F);
+    int first = 84, count = 256;   // nodes of the level before, nodes of the level
+    while (true) {
+        if (m < count)
+            for (int a = 0; a < 6; ++a) q[6 * (first + m) + a] = box[m][a];
+        if (count == 4) break;
+        __syncthreads();
+        float u[6];
+        count >>= 2;
+        first -= count;
+        if (m < count)
+            for (int a = 0; a < 6; ++a) {
+                u[a] = box[4 * m][a];
+                for (int k = 1; k < 4; ++k) u[a] = a < 3 ? fminf(u[a], box[4 * m + k][a]) : fmaxf(u[a], box[4 * m + k][a]);
+            }
+        __syncthreads();
+        if (m < count)
+            for (int a = 0; a < 6; ++a) box[m][a] = u[a];
+        __syncthreads();
+    }
+}
+
+cudaError_t launch_quad_boxes(const DScene& S, int n_patches, float* out, cudaStream_t st) {
+    if (n_patches <= 0) return cudaSuccess;
+    k_quad_boxes<<<static_cast<unsigned>(n_patches), 256, 0, st>>>(S, out);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_leaf_records(const DScene& S, int n_slots, float4* out, cudaStream_t st) {
