@@ -428,7 +428,9 @@ typedef struct bbrt_tuning {
     int advance_shape;        /* k_advance launch shape, threads x blocks per SM: 0 = 128x3, 1 = 256x2,
                                  2 = 128x4, 3 = 512x1 (default), 4 = 768x1, 5 = 1024x1, 6 = 384x1 */
     int warp_stage1;          /* no effect: a patch's stage 1 always runs by the whole warp */
-    int order_rays;           /* 1 (default): bucket rays by direction and origin before round 0 */
+    int order_rays;           /* 1 (default): bucket rays by direction and origin before round 0 (a scene whose
+                                 schedule was never set or autotuned takes them as they come where that
+                                 is faster) */
     int warp_tail;            /* 1 (default): the tail one warp per ray, else one thread per ray */
     long long wave_tail;      /* rays still waiting when the tail takes over (4096) */
     long long wave_min_rays;  /* smaller batches run one ray per warp to the end (8192; a scene whose schedule
@@ -452,7 +454,8 @@ BBRT_API int bbrt_scene_get_tuning(bbrt_scene_t scene, bbrt_tuning* out);
 BBRT_API int bbrt_scene_set_tuning(bbrt_scene_t scene, const bbrt_tuning* tuning);
 /* Times candidate schedules on the given rays (host arrays; the scene's
  * current precision and guess modes), by coordinate descent over the launch
- * shape, then the tail size, then graph-launched vs host-driven rounds, `trials` timed traces each after one untimed
+ * shape, then the tail size, then ordered or unordered rays, then graph-launched vs
+ * host-driven rounds, `trials` timed traces each after one untimed
  * one; keeps the fastest in the scene and returns it with its mean device
  * time per trace. */
 BBRT_API int bbrt_scene_autotune(bbrt_scene_t scene, const double* origins, const double* dirs, long long n,
