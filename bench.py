@@ -20,8 +20,8 @@ value     bounces of all rays / device time of one step of the learned-guess
 e2e       the same metric through bbrt_trace with pinned host buffers: the
           host->device copy of the rays and the device->host copy of the
           per-ray results are inside the timed region.
-roofline  the dominant kernel (k_advance: BVH traversal and stage 1, the same
-          in every form) against the pipe peaks measured in this process.
+roofline  the advance kernels (BVH traversal and stage 1: k_walk and k_stage1,
+          or k_advance; the same in every form) against the pipe peaks measured in this process.
 cpu_baseline  the reference's own OpenMP trace loop (oracle/_ref), or the
           oracle port when the reference was not built, on a bounded sample
           of the same rays on all host cores (rank 0, N = 1 only).
@@ -172,8 +172,9 @@ PROFILE_TRAFFIC = os.path.join(ROOT, "profiles", "k_advance_traffic.json")
 
 
 def advance_roofline(st, fp64_peak, fp32_peak, l2_peak):
-    """Roofline of the dominant kernel, k_advance, from its own counters and its
-    own device time (CUDA events around each launch inside the library).
+    """Roofline of the advance kernels of a round (k_walk and k_stage1, or
+    k_advance, which the line's key names for both), from their own counters and
+    device time (CUDA events around each round's launches inside the library).
 
     Work per unit:
       BVH node test, FP32    16 FP32 FLOP (6 differences, 6 products, 4
@@ -208,17 +209,17 @@ def advance_roofline(st, fp64_peak, fp32_peak, l2_peak):
     traffic = None
     if os.path.exists(PROFILE_TRAFFIC):
         prof = json.load(open(PROFILE_TRAFFIC))
-        # scale the captured launch's DRAM bytes to a whole step of k_advance launches by the work done
+        # scale the captured launches' DRAM bytes to a whole step's rounds by the work done
         if prof.get("node_tests"):
             traffic = prof["dram_bytes"] * nodes / prof["node_tests"] / max(1, st["rounds"])
     return {"bound": best, "achieved": a, "peak": p, "unit": u, "frac": a / p, "traffic": traffic,
             "kernel": "k_advance", "launches_per_step": int(st["rounds"]),
             "pipes": {k: {"achieved": v[0], "peak": v[1], "unit": v[2], "frac": v[0] / v[1]} for k, v in pipes.items()},
-            "note": "algorithmic work of the k_advance launches of one step (device counters) over their summed "
-                    "CUDA-event time; peaks: FP64/FP32 FMA and L2-resident reads measured in this process "
+            "note": "algorithmic work of the advance kernels (k_walk and k_stage1) of one step (device counters) over "
+                    "their summed CUDA-event time; peaks: FP64/FP32 FMA and L2-resident reads measured in this process "
                     f"(bbrt_measure_pipe_peak), of measured; HBM {HBM_PEAK_GBS:.0f} GB/s, of {HBM_PEAK_SOURCE} "
                     f"({'MEASURED_PEAKS.json' if HBM_PEAK_SOURCE == 'measured' else 'no MEASURED_PEAKS.json: the pool fallback'}); the exact FP64 "
-                    "path runs unfused mul/add (half the FMA peak at most); traffic per launch from the ncu "
+                    "path runs unfused mul/add (half the FMA peak at most); traffic per round from the ncu "
                     "capture in profiles/, scaled by node tests"}
 
 

@@ -418,8 +418,7 @@ BBRT_API int bbrt_trace_batch(const bbrt_scene_t* scenes, int n_scenes, const do
  *
  * The schedule changes only the order and grouping of work, never a result
  * (every schedule gives the same bits; GPU-tested).  A scene starts with the
- * library defaults (environment overrides BBRT_ADV_SHAPE, BBRT_WARP_S1,
- * BBRT_ORDER_RAYS, BBRT_WARP_TAIL, BBRT_WAVE_TAIL, BBRT_WAVE_MIN, BBRT_GRAPH
+ * library defaults (environment overrides BBRT_ADV_SHAPE, BBRT_ORDER_RAYS, BBRT_WARP_TAIL, BBRT_WAVE_TAIL, BBRT_WAVE_MIN, BBRT_GRAPH
  * are read once per process; so are BBRT_NODE_F32 (0: FP64 BVH node tests
  * only), BBRT_ADAPT_LANES (0: a small round's warps take 32 rays each) and
  * BBRT_NEWTON_GROUP_MAX (largest Newton round solved 8 lanes per request,
@@ -438,11 +437,11 @@ typedef struct bbrt_tuning {
     int graph_rounds;         /* 1 (default): the whole wavefront trace is one CUDA graph launch whose
                                  round loop is a device-side conditional node (no host wait per round;
                                  one graph per argument set, kept for reuse); 0: rounds driven by the host */
-    long long watchdog_cycles;  /* a k_advance launch that runs longer than this many SM clock cycles
+    long long watchdog_cycles;  /* a round's launch (k_walk, k_stage1, k_advance) that runs longer than this many SM clock cycles
                                    stops, and the call returns BBRT_ERR_KERNEL ("watchdog") instead of
                                    holding the GPU; 0 = the default, 2^35 (about 17 s at 1.97 GHz; a
-                                   round takes milliseconds).  Checked on a warp's first loop
-                                   iteration and every 1024th after it. */
+                                   round takes milliseconds).  Checked by every warp as it goes on
+                                   to its next rays (k_advance: every 256th loop iteration). */
     long long mma_wait_cycles;  /* a tensor-core completion wait of the learned-guess kernels gives up
                                    after this many SM clock cycles (it then waits once more, with the
                                    default bound, for the MMAs in flight, frees its tensor memory and
