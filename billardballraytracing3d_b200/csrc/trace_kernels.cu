@@ -204,8 +204,9 @@ __global__ void __launch_bounds__(128, 4) k_newton_auto(DScene S, TraceArgs A, W
 }
 
 // Finishes rays from their saved state with inline queries (the tail of a
-// wavefront trace, and rays whose query overflowed the resolved list).  The
-// current bounce's query restarts from the root, so the result is the same.
+// wavefront trace, and rays whose query overflowed the resolved list), or the
+// single queries of such a round.  The current query restarts from the root, so
+// the result is the same.
 __global__ void __launch_bounds__(128) k_resume(DScene S, TraceArgs A, WaveArgs W, const NewtonRequest* reqs,
                                                 const int* rays, long long n) {
     if (W.count_dev) {
@@ -219,11 +220,15 @@ __global__ void __launch_bounds__(128) k_resume(DScene S, TraceArgs A, WaveArgs 
         const long long i = reqs ? reqs[slot].ray : rays[slot];
         int nres;
         RayCtx r = load_ray(A, W, i, nres);
-        run_ray(S, A, i, r, ctr, tally.queries);
-        add_ray_work(A, i, ctr);
-        finish_ray(A, i, r);
-        tally.bounces += r.bounces;
-        tally.hist[r.status]++;
+        if (A.query_out) {
+            write_hit(static_cast<bbrt_hit*>(A.query_out) + i, bvh_query(S, r.o, r.d, A.cull, ctr, false, r.member));
+        } else {
+            run_ray(S, A, i, r, ctr, tally.queries);
+            add_ray_work(A, i, ctr);
+            finish_ray(A, i, r);
+            tally.bounces += r.bounces;
+            tally.hist[r.status]++;
+        }
     }
     flush_stats(A, ctr, tally, true);
 }

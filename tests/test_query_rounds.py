@@ -1,0 +1,42 @@
+"""Batches of single queries that run as wavefront rounds: every schedule gives
+the oracle's records, bit for bit, and the same as a warp per query."""
+import numpy as np
+import pytest
+
+import oracle
+from billardballraytracing3d_b200 import _capi as C
+from billardballraytracing3d_b200 import api, scenes
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ("object", "status", "err_object", "t", "point", "normal", "uv", "err_value")
+
+
+@pytest.fixture(scope="module")
+def nested(built):
+    """Concentric spheres (queries with many stage-1 hits) and 9,001 rays at
+    them; every fifth direction is longer than a unit, so its query is not
+    culled and leaves the rounds through the overflow list."""
+    patches = []
+    for k, r in enumerate((1.0, 1.4, 1.9, 2.5, 3.2)):
+        patches += scenes.obstacle_patches(k, (0.0, 0.0, 0.0), (r, r, r), None, m=2, n_nodes=5)
+    rng = np.random.Generator(np.random.PCG64(3))
+    o = rng.normal(size=(9001, 3))
+    o = 6.0 * o / np.linalg.norm(o, axis=1, keepdims=True)
+    d = -o + rng.normal(size=(9001, 3)) * 0.8
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    d[::5] *= 2.0
+    cfg = C.default_config(coarse_grid_n=9, newton_tol=1e-12)
+    return patches, cfg, o, d, oracle.Oracle(patches, config=cfg).intersect(o, d)
+
+
+@pytest.mark.parametrize("graph_rounds", [1, 0])
+@pytest.mark.parametrize("warp_tail", [1, 0])
+@pytest.mark.parametrize("wave_tail", [0, 4096, 1000000])
+def test_schedules_do_not_change_query_results(nested, graph_rounds, warp_tail, wave_tail):
+    patches, cfg, o, d, ref = nested
+    sc = api.Scene(patches, config=cfg)
+    sc.tuning(graph_rounds=graph_rounds, warp_tail=warp_tail, wave_tail=wave_tail, wave_min_rays=1)
+    got = sc.intersect(o, d)
+    for k in KEYS:
+        assert np.array_equal(got[k], ref[k], equal_nan=True), k
