@@ -192,6 +192,8 @@ struct bbrt_scene {
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[4] = { nullptr, nullptr, nullptr, nullptr };
+    cudaEvent_t busy = nullptr;     // the end of the last trace that returned with its work in flight ...
+    bool in_flight = false;         // ... where there was one
     std::vector<void*> allocs;
     long long device_bytes = 0;
     DevBuf stats, work, in_o, in_d, o_status, o_bounce, o_dir, o_end, o_hobj, o_hpt, o_huv, o_eobj, o_eval,
@@ -252,6 +254,7 @@ struct bbrt_scene {
                            &guess.out, &guess.rows })
             b->release();
         if (wave_ctr_host) cudaFreeHost(wave_ctr_host);
+        if (busy) cudaEventDestroy(busy);
         for (auto& e : slot_ev)
             if (e) cudaEventDestroy(e);
         for (WaveGraph& g : wgraphs) {
@@ -374,6 +377,7 @@ int ensure_device(bbrt_scene* s) {
     BBRT_CUDA(bbrt::noalloc_prepare());
     for (auto& e : s->ev) BBRT_CUDA(cudaEventCreate(&e));
     for (auto& e : s->kev) BBRT_CUDA(cudaEventCreate(&e));
+    BBRT_CUDA(cudaEventCreateWithFlags(&s->busy, cudaEventDisableTiming));
     s->device_ready = true;
     return BBRT_OK;
 }
@@ -1125,6 +1129,10 @@ long long wave_min(const bbrt_scene* s) {
     return plain && !tuning().wave_min_set ? 32768 : tuning().wave_min_rays;
 }
 
+// Whether a trace of n rays on device arrays has finished when its call
+// returns: from the schedule's wavefront size on, whichever kernels run it.
+bool waits_for_trace(const bbrt_scene* s, long long n) { return n >= scene_tuning(s).wave_min_rays; }
+
 // The k_advance watchdog and the tensor-core wait bound of a schedule
 // (0 in the schedule: the defaults).
 long long watchdog_cycles(const bbrt_tuning& T) { return T.watchdog_cycles > 0 ? T.watchdog_cycles : 1LL << 35; }
@@ -1579,8 +1587,28 @@ int check_guess_waits(bbrt_scene* s, cudaStream_t st) {
     return BBRT_OK;
 }
 
-// Launches the trace kernel on device arrays.  hit_counts (device, may be
-// null) receives per-object counts for bounces with index >= count_from.
+// Orders `st` after the scene's last trace, whose work may still run on another
+// stream: all traces of a scene hand out rays through one counter and count in
+// one statistics block, which each call clears.  A stream under capture cannot
+// wait for work outside it: ordering its replays is the caller's.
+int after_last_trace(bbrt_scene* s, cudaStream_t st) {
+    if (!s->in_flight) return BBRT_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    BBRT_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap == cudaStreamCaptureStatusNone) BBRT_CUDA(cudaStreamWaitEvent(st, s->busy, 0));
+    return BBRT_OK;
+}
+
+// The call returns with its trace in flight on `st` (see after_last_trace).
+int leave_in_flight(bbrt_scene* s, cudaStream_t st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    BBRT_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return BBRT_OK;
+    BBRT_CUDA(cudaEventRecord(s->busy, st));
+    s->in_flight = true;
+    return BBRT_OK;
+}
+
 // Trace arguments of one call and the per-call resets (statistics, ray
 // counter, per-kernel timing); records the call's start event.
 int prepare_trace(bbrt_scene* s, const double* d_o, const double* d_d, long long n, int max_bounces,
@@ -1615,6 +1643,8 @@ int prepare_trace(bbrt_scene* s, const double* d_o, const double* d_d, long long
     A.sample_cap_pos = s->rec_cap_pos;
     A.sample_cap_neg = s->rec_cap_neg;
     A.ray_member = s->ray_member;
+    const int rc = after_last_trace(s, st);
+    if (rc) return rc;
     if (want_stats) BBRT_CUDA(cudaMemsetAsync(s->stats.p, 0, sizeof(long long) * bbrt::ST_COUNT, st));
     BBRT_CUDA(cudaMemsetAsync(s->work.p, 0, sizeof(unsigned long long), st));
     if (learned_trace(s)) {
@@ -1660,10 +1690,11 @@ int run_trace_device(bbrt_scene* s, const double* d_o, const double* d_d, long l
         if (rc) return rc;
     }
     rc = complete_trace(s, st, want_stats, host_stats, kernel_ms);
-    if (!rc && graph.on) {
-        // a graph-launched trace: one host wait, for its device-side bounds
+    // one host wait: for a graph's device-side bounds, and because callers read
+    // the results of a trace of this size when the call returns
+    if (!rc && waits_for_trace(s, n)) {
         BBRT_CUDA(cudaEventSynchronize(s->ev[1]));
-        rc = check_wave_graph(s, graph);
+        if (graph.on) rc = check_wave_graph(s, graph);
     }
     if (!rc && n >= wave_min(s)) rc = check_guess_waits(s, st);
     return rc;
@@ -1988,6 +2019,7 @@ BBRT_API int bbrt_trace(bbrt_scene_t s, const double* origins, const double* dir
                               stats ? &kms : nullptr);
         s->time_kernels = false;
         if (rc) return rc;
+        if (!waits_for_trace(s, n) && (rc = leave_in_flight(s, st))) return rc;
         if (stats) {
             BBRT_CUDA(cudaStreamSynchronize(st));
             fill_stats(s, hs, n, kms, kms, stats);

@@ -298,7 +298,12 @@ BBRT_API int  bbrt_intersect(bbrt_scene_t scene, const double* origins, const do
  * for n rays in one call (the batch form of run(), :143-150).  Directions
  * need not be normalised.  With flags & BBRT_DEVICE_PTRS every array in the
  * call is a device pointer; otherwise host pointers are staged through the
- * scene's device buffers inside the call. */
+ * scene's device buffers inside the call.
+ * With device pointers a trace of at least wave_min_rays rays (bbrt_tuning; 8192)
+ * or with stats has finished when the call returns; a smaller one is in flight on
+ * `stream` and its results are ready in that stream's order.  Any later trace on
+ * the handle, on whatever stream, starts after it.  (A call under stream capture
+ * is ordered neither way: order its replays against the handle's other calls.) */
 BBRT_API int  bbrt_trace(bbrt_scene_t scene, const double* origins, const double* dirs,
                          long long n, int max_bounces, int flags,
                          const bbrt_trace_out* out, bbrt_trace_stats* stats, void* stream);
