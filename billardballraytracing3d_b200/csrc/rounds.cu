@@ -257,9 +257,10 @@ __global__ void __launch_bounds__(kWalkThreads, 4) k_walk(DScene S, TraceArgs A,
         if (ask) W.req[a_ask + __popc(m_ask & before)] = rq;
         if (over) W.overflow[a_over + __popc(m_over & before)] = i;
         if (listed) W.listed[a_list + __popc(m_list & before)] = i;
-        // a launch that runs far past any real round gives up (see advance.cu)
-        if (clock64() - t_start > W.watchdog_cycles) {
-            atomicOr(&W.counters[3], 1u);
+        // a launch that runs far past any real round gives up (see advance.cu), the
+        // whole warp at once: the lanes' clocks need not agree
+        if (__any_sync(kFull, clock64() - t_start > W.watchdog_cycles)) {
+            if (lane == 0) atomicOr(&W.counters[3], 1u);
             break;
         }
     }
