@@ -9,10 +9,8 @@
 //   BounceMapDriver::run                                  BounceMapDriver.hpp:103-259
 //   SurfacePatch::load_patch_file / sample_grid           SurfacePatch.hpp:313-371, :199-242
 #include <cuda_runtime.h>
-#include <omp.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -35,6 +33,7 @@
 #include "scene_compile.h"
 #include "scene_set.h"
 #include "scene_host.hpp"
+#include "host_io.hpp"
 
 namespace bbrt {
 cudaError_t launch_rays(const DScene& S, const TraceArgs& A, const WaveArgs& W, const NewtonRequest* reqs, const int* rays,
@@ -79,6 +78,8 @@ cudaError_t launch_bounce_reduce(const int* status, const int* bounces, long lon
 
 namespace {
 
+using bbrt::DevBuf;
+
 thread_local std::string g_error;
 
 int fail(int code, const std::string& msg) {
@@ -92,89 +93,6 @@ int fail(int code, const std::string& msg) {
         if (e_ != cudaSuccess)                                                            \
             return fail(BBRT_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
-
-// A grow-only device buffer, freed when it goes out of scope.
-struct DevBuf {
-    void* p = nullptr;
-    size_t bytes = 0;
-    DevBuf() = default;
-    DevBuf(const DevBuf&) = delete;
-    DevBuf& operator=(const DevBuf&) = delete;
-    ~DevBuf() { release(); }
-    cudaError_t ensure(size_t n) {
-        if (n <= bytes) return cudaSuccess;
-        if (p) cudaFree(p);
-        p = nullptr;
-        bytes = 0;
-        cudaError_t e = cudaMalloc(&p, n);
-        if (e == cudaSuccess) bytes = n;
-        return e;
-    }
-    void release() {
-        if (p) cudaFree(p);
-        p = nullptr;
-        bytes = 0;
-    }
-};
-
-// Pinned host memory for calls on host arrays (HostIo), shared by the scenes:
-// pinning 1 MB takes about a millisecond, more than a small call.  A call
-// borrows a block and gives it back; at most kKeep of each kind stay for the
-// next ones, and all are freed with the last scene.
-class PinPool {
-public:
-    static constexpr int kSlots = 16;
-    static constexpr size_t kSlot = 512 << 10;
-    static constexpr size_t kBytes[2] = { 1 << 20, kSlots * kSlot };   // a small call's block; slots of a large one
-    static PinPool& get() {
-        static PinPool* p = new PinPool;   // outlives the last scene
-        return *p;
-    }
-    cudaError_t take(int kind, char** out) {
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            if (n_[kind] > 0) {
-                *out = free_[kind][--n_[kind]];
-                return cudaSuccess;
-            }
-        }
-        return cudaHostAlloc(reinterpret_cast<void**>(out), kBytes[kind], cudaHostAllocPortable);
-    }
-    void give(int kind, char* p) {
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            if (users_ > 0 && n_[kind] < kKeep) {
-                free_[kind][n_[kind]++] = p;
-                return;
-            }
-        }
-        cudaFreeHost(p);
-    }
-    // A scene's share in the pool's life.
-    struct User {
-        User() {
-            PinPool& p = get();
-            std::lock_guard<std::mutex> g(p.mu_);
-            ++p.users_;
-        }
-        ~User() {
-            PinPool& p = get();
-            std::lock_guard<std::mutex> g(p.mu_);
-            if (--p.users_ > 0) return;
-            for (int k = 0; k < 2; ++k)
-                while (p.n_[k] > 0) cudaFreeHost(p.free_[k][--p.n_[k]]);
-        }
-        User(const User&) = delete;
-        User& operator=(const User&) = delete;
-    };
-
-private:
-    static constexpr int kKeep = 2;
-    std::mutex mu_;
-    char* free_[2][kKeep] = {};
-    int n_[2] = { 0, 0 };
-    int users_ = 0;
-};
 
 }  // namespace
 
@@ -198,8 +116,8 @@ struct bbrt_scene {
     long long device_bytes = 0;
     DevBuf stats, work, in_o, in_d, o_status, o_bounce, o_dir, o_end, o_hobj, o_hpt, o_huv, o_eobj, o_eval,
         counts, hits, wave, wave_ctr, o_work, order, order_ws, io;
-    cudaEvent_t slot_ev[PinPool::kSlots] = {};   // one per copying thread of HostIo
-    PinPool::User pin_user;
+    cudaEvent_t slot_ev[bbrt::PinPool::kSlots] = {};   // one per copying thread of HostIo
+    bbrt::PinPool::User pin_user;
     unsigned int* wave_ctr_host = nullptr;   // pinned copy of the round counters
     // per-launch timing of calls that collect statistics
     static constexpr int kTimerEvents = 96;
@@ -838,141 +756,6 @@ int create_from_files(const std::vector<std::string>& paths, const bbrt_config* 
 cudaStream_t pick_stream(bbrt_scene* s, void* stream) {
     return stream ? static_cast<cudaStream_t>(stream) : s->stream;
 }
-
-// The host arrays of one call on their way to the device and back.  A copy
-// from or to pageable memory goes through the driver's staging on one thread
-// (about 4 GB/s into pages that are not yet there) and costs several
-// microseconds however small, so, by the call's bytes:
-//   at most kZeroCopy    the kernels read and write a pinned block, no copies
-//                        (96 queries: 58 us, 67 with one copy each way, 75
-//                        with the driver's staging; 61 recorded paths 142,
-//                        148, 258 us);
-//   at most kOneCopy     one copy each way between that block and the device;
-//   more                 chunks through pinned slots by several threads, which
-//                        also spread the page faults of the caller's arrays
-//                        (262,147 recorded paths, 97 MB of results: 24 ms with
-//                        the driver's staging, 8.4 ms this way on 16 cores);
-//                        arrays that are pinned already are copied directly.
-struct HostIo {
-    static constexpr size_t kZeroCopy = 64 << 10, kOneCopy = PinPool::kBytes[0], kChunk = PinPool::kSlot;
-    static constexpr int kMaxArrays = 12, kMaxThreads = PinPool::kSlots;
-    struct Array {
-        char* host;
-        size_t bytes, off;
-        bool in, direct;   // direct: pinned memory, copied as it is
-    };
-    bbrt_scene* s;
-    cudaStream_t st;
-    Array a[kMaxArrays];
-    int n = 0;
-    size_t in_bytes = 0, total = 0;
-    char* base = nullptr;   // the block the kernels use
-    char* held[2] = { nullptr, nullptr };   // pinned memory borrowed from the pool
-
-    HostIo(bbrt_scene* s_, cudaStream_t st_) : s(s_), st(st_) {}
-    HostIo(const HostIo&) = delete;
-    HostIo& operator=(const HostIo&) = delete;
-    ~HostIo() {
-        if (!held[0] && !held[1]) return;
-        if (!done) cudaStreamSynchronize(st);   // a failed call: nothing may still use the block
-        for (int k = 0; k < 2; ++k)
-            if (held[k]) PinPool::get().give(k, held[k]);
-    }
-
-    // Inputs first, then outputs (a null array is skipped); at(i) after open().
-    int add(const void* host, size_t bytes, bool in) {
-        if (!host || bytes == 0) return -1;
-        a[n] = { static_cast<char*>(const_cast<void*>(host)), bytes, total, in, false };
-        total += (bytes + 255) & ~static_cast<size_t>(255);
-        if (in) in_bytes = total;
-        return n++;
-    }
-    template <class T>
-    T* at(int i) const { return i < 0 ? nullptr : reinterpret_cast<T*>(base + a[i].off); }
-
-    int open() {
-        if (total > kZeroCopy) {
-            BBRT_CUDA(s->io.ensure(total));
-            base = static_cast<char*>(s->io.p);
-        }
-        if (total > kOneCopy)
-            for (int k = 0; k < n; ++k) {
-                cudaPointerAttributes pa;
-                if (cudaPointerGetAttributes(&pa, a[k].host) == cudaSuccess)
-                    a[k].direct = pa.type == cudaMemoryTypeHost || pa.type == cudaMemoryTypeDevice;
-                else
-                    cudaGetLastError();
-            }
-        if (in_bytes > kOneCopy || (n > 0 && a[0].direct)) return bulk(true);
-        BBRT_CUDA(PinPool::get().take(0, &held[0]));
-        if (total <= kZeroCopy) base = held[0];
-        for (int k = 0; k < n; ++k)
-            if (a[k].in) std::memcpy(held[0] + a[k].off, a[k].host, a[k].bytes);
-        if (total > kZeroCopy && in_bytes) BBRT_CUDA(cudaMemcpyAsync(base, held[0], in_bytes, cudaMemcpyHostToDevice, st));
-        return BBRT_OK;
-    }
-
-    // The results are in the caller's arrays when this returns.
-    int close() {
-        if (total > kOneCopy) {
-            const int rc = bulk(false);
-            if (rc) return rc;
-        } else if (total > kZeroCopy && total > in_bytes) {
-            BBRT_CUDA(cudaMemcpyAsync(held[0] + in_bytes, base + in_bytes, total - in_bytes, cudaMemcpyDeviceToHost, st));
-        }
-        BBRT_CUDA(cudaStreamSynchronize(st));
-        done = true;
-        if (total <= kOneCopy)
-            for (int k = 0; k < n; ++k)
-                if (!a[k].in) std::memcpy(a[k].host, held[0] + a[k].off, a[k].bytes);
-        return BBRT_OK;
-    }
-
-private:
-    bool done = false;
-
-    int bulk(bool up) {
-        const cudaMemcpyKind kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-        size_t first[kMaxArrays + 1] = {};   // first chunk of each array that is staged
-        for (int k = 0; k < n; ++k) {
-            const bool staged = a[k].in == up && !a[k].direct;
-            first[k + 1] = first[k] + (staged ? (a[k].bytes + kChunk - 1) / kChunk : 0);
-            if (a[k].in == up && a[k].direct) {
-                char* dev = base + a[k].off;
-                BBRT_CUDA(cudaMemcpyAsync(up ? dev : a[k].host, up ? a[k].host : dev, a[k].bytes, kind, st));
-            }
-        }
-        const size_t chunks = first[n];
-        if (chunks == 0) return BBRT_OK;
-        if (!held[1]) BBRT_CUDA(PinPool::get().take(1, &held[1]));
-        for (auto& e : s->slot_ev)
-            if (!e) BBRT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        const int threads = static_cast<int>(std::min<size_t>(chunks, std::min(kMaxThreads, omp_get_max_threads())));
-        std::atomic<size_t> next{ 0 };
-        std::atomic<int> err{ cudaSuccess };
-        #pragma omp parallel num_threads(threads)
-        {
-            const int me = omp_get_thread_num();
-            char* slot = held[1] + kChunk * me;
-            cudaError_t e = cudaSetDevice(s->device);
-            for (size_t c = next++; e == cudaSuccess && c < chunks; c = next++) {
-                int k = 0;
-                while (c >= first[k + 1]) ++k;
-                const size_t at = (c - first[k]) * kChunk, bytes = std::min(kChunk, a[k].bytes - at);
-                char *host = a[k].host + at, *dev = base + a[k].off + at;
-                if (up) std::memcpy(slot, host, bytes);
-                e = cudaMemcpyAsync(up ? dev : slot, up ? slot : dev, bytes, kind, st);
-                if (e == cudaSuccess) e = cudaEventRecord(s->slot_ev[me], st);
-                if (e == cudaSuccess) e = cudaEventSynchronize(s->slot_ev[me]);
-                if (e == cudaSuccess && !up) std::memcpy(host, slot, bytes);
-            }
-            if (e != cudaSuccess) err = e;
-        }
-        if (err != cudaSuccess)
-            return fail(BBRT_ERR_CUDA, std::string("host array copy: ") + cudaGetErrorString(static_cast<cudaError_t>(err.load())));
-        return BBRT_OK;
-    }
-};
 
 void fill_stats(bbrt_scene* s, const long long* st, long long n, float kernel_ms, float total_ms,
                 bbrt_trace_stats* out) {
@@ -1978,10 +1761,10 @@ BBRT_API int bbrt_intersect(bbrt_scene_t s, const double* origins, const double*
         return BBRT_OK;
     }
     const size_t vb = sizeof(double) * 3 * static_cast<size_t>(n);
-    HostIo io(s, st);
+    bbrt::HostIo io(s->io, s->slot_ev, s->device, st);
     const int o = io.add(origins, vb, true), d = io.add(dirs, vb, true);
     const int h = io.add(out, sizeof(bbrt_hit) * static_cast<size_t>(n), false);
-    if ((rc = io.open())) return rc;
+    BBRT_CUDA(io.open());
     Q.origins = io.at<double>(o);
     Q.dirs = io.at<double>(d);
     Q.out = io.at<bbrt_hit>(h);
@@ -1992,7 +1775,8 @@ BBRT_API int bbrt_intersect(bbrt_scene_t s, const double* origins, const double*
     } else {
         BBRT_CUDA(mode == BBRT_QUERY_BVH ? bbrt::launch_query_warp(s->dev, Q, s->sm_count, st) : bbrt::launch_query(s->dev, Q, st));
     }
-    return io.close();
+    BBRT_CUDA(io.close());
+    return BBRT_OK;
 }
 
 BBRT_API int bbrt_trace(bbrt_scene_t s, const double* origins, const double* dirs, long long n, int max_bounces,
@@ -2029,7 +1813,7 @@ BBRT_API int bbrt_trace(bbrt_scene_t s, const double* origins, const double* dir
     // host arrays
     const size_t N = static_cast<size_t>(n), K = out ? static_cast<size_t>(out->record_bounces) : 0;
     BBRT_CUDA(cudaEventRecord(s->ev[2], st));
-    HostIo io(s, st);
+    bbrt::HostIo io(s->io, s->slot_ev, s->device, st);
     const int i_o = io.add(origins, sizeof(double) * 3 * N, true), i_d = io.add(dirs, sizeof(double) * 3 * N, true);
     int i_out[10] = { -1, -1, -1, -1, -1, -1, -1, -1, -1, -1 };
     if (out) {
@@ -2040,7 +1824,7 @@ BBRT_API int bbrt_trace(bbrt_scene_t s, const double* origins, const double* dir
                                    sizeof(int) * N, sizeof(double) * 2 * N, sizeof(long long) * 4 * N };
         for (int k = 0; k < 10; ++k) i_out[k] = io.add(host[k], bytes[k], false);
     }
-    if ((rc = io.open())) return rc;
+    BBRT_CUDA(io.open());
     bbrt_trace_out dev{};
     if (out) {
         dev.record_bounces = out->record_bounces;
@@ -2060,7 +1844,7 @@ BBRT_API int bbrt_trace(bbrt_scene_t s, const double* origins, const double* dir
                           counters, hs, nullptr);
     s->time_kernels = false;
     if (rc) return rc;
-    if ((rc = io.close())) return rc;
+    BBRT_CUDA(io.close());
     if (stats) {
         BBRT_CUDA(cudaEventRecord(s->ev[3], st));
         BBRT_CUDA(cudaEventSynchronize(s->ev[3]));
