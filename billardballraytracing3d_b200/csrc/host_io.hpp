@@ -39,38 +39,39 @@ struct DevBuf {
 
 // Pinned host memory for calls on host arrays (HostIo), shared by the scenes:
 // pinning 1 MB takes about a millisecond, more than a small call.  A call
-// borrows a block and gives it back; at most kKeep of each kind stay for the
-// next ones, and all are freed with the last scene.
+// borrows a block and gives it back; there are at most kMax of each kind, and
+// all are freed with the last scene.  A call that gets none (all are out, or
+// the system pins no more) copies without.
 class PinPool {
 public:
     static constexpr int kSlots = 16;
     static constexpr size_t kSlot = 512 << 10;
     static constexpr size_t kBytes[2] = { 1 << 20, kSlots * kSlot };   // a small call's block; slots of a large one
+    static constexpr int kMax[2] = { 16, 4 };
     static PinPool& get() {
         static PinPool* p = new PinPool;   // outlives the last scene
         return *p;
     }
-    cudaError_t take(int kind, char** out) {
+    // A block, or null.
+    char* take(int kind) {
         {
             std::lock_guard<std::mutex> g(mu_);
-            if (n_[kind] > 0) {
-                *out = free_[kind][--n_[kind]];
-                return cudaSuccess;
-            }
+            if (n_[kind] > 0) return free_[kind][--n_[kind]];
+            if (made_[kind] == kMax[kind]) return nullptr;
+            ++made_[kind];
         }
-        return cudaHostAlloc(reinterpret_cast<void**>(out), kBytes[kind], cudaHostAllocPortable);
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, kBytes[kind], cudaHostAllocPortable) == cudaSuccess) return static_cast<char*>(p);
+        cudaGetLastError();
+        std::lock_guard<std::mutex> g(mu_);
+        --made_[kind];
+        return nullptr;
     }
     void give(int kind, char* p) {
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            if (users_ > 0 && n_[kind] < kKeep) {
-                free_[kind][n_[kind]++] = p;
-                return;
-            }
-        }
-        cudaFreeHost(p);
+        std::lock_guard<std::mutex> g(mu_);
+        free_[kind][n_[kind]++] = p;
     }
-    // A scene's share in the pool's life.
+    // A scene's share in the pool's life; its calls have ended when it goes.
     struct User {
         User() {
             PinPool& p = get();
@@ -82,17 +83,16 @@ public:
             std::lock_guard<std::mutex> g(p.mu_);
             if (--p.users_ > 0) return;
             for (int k = 0; k < 2; ++k)
-                while (p.n_[k] > 0) cudaFreeHost(p.free_[k][--p.n_[k]]);
+                for (; p.n_[k] > 0; --p.made_[k]) cudaFreeHost(p.free_[k][--p.n_[k]]);
         }
         User(const User&) = delete;
         User& operator=(const User&) = delete;
     };
 
 private:
-    static constexpr int kKeep = 2;
     std::mutex mu_;
-    char* free_[2][kKeep] = {};
-    int n_[2] = { 0, 0 };
+    char* free_[2][16] = {};
+    int n_[2] = { 0, 0 }, made_[2] = { 0, 0 };
     int users_ = 0;
 };
 
@@ -111,7 +111,8 @@ private:
 //                        results: 24 ms with the driver's staging, 8.4 ms this
 //                        way on 16 cores); pinned arrays are copied directly.
 // Array by array too, at any size, where an array is device memory (its copy is
-// CUDA's to make or to refuse: the host cannot read it).
+// CUDA's to make or to refuse: the host cannot read it), and with the driver's
+// staging where the pool has no block.
 struct HostIo {
     static constexpr size_t kZeroCopy = 64 << 10, kOneCopy = PinPool::kBytes[0], kChunk = PinPool::kSlot;
     static constexpr int kMaxArrays = 12, kMaxThreads = PinPool::kSlots;
@@ -164,8 +165,8 @@ struct HostIo {
             by_array = by_array || a[k].direct;
         }
         if (!by_array) {
-            const cudaError_t e = PinPool::get().take(0, &held[0]);
-            if (e != cudaSuccess) return e;
+            held[0] = PinPool::get().take(0);
+            by_array = !held[0];
         }
         if (!by_array && total <= kZeroCopy) {
             base = held[0];
@@ -205,17 +206,14 @@ private:
         for (int k = 0; k < n; ++k)
             first[k + 1] = first[k] + (a[k].in == up && !a[k].direct ? (a[k].bytes + kChunk - 1) / kChunk : 0);
         const size_t chunks = first[n];
-        if (chunks && !held[1]) {
-            const cudaError_t e = PinPool::get().take(1, &held[1]);
-            if (e != cudaSuccess) return e;
-        }
+        if (chunks && !held[1]) held[1] = PinPool::get().take(1);
         for (int k = 0; k < n; ++k) {
-            if (a[k].in != up || !a[k].direct) continue;
+            if (a[k].in != up || (!a[k].direct && held[1])) continue;
             char* dev = base + a[k].off;
             const cudaError_t e = cudaMemcpyAsync(up ? dev : a[k].host, up ? a[k].host : dev, a[k].bytes, kind, st);
             if (e != cudaSuccess) return e;
         }
-        if (chunks == 0) return cudaSuccess;
+        if (chunks == 0 || !held[1]) return cudaSuccess;
         for (int k = 0; k < kMaxThreads; ++k) {
             if (slot_ev[k]) continue;
             const cudaError_t e = cudaEventCreateWithFlags(&slot_ev[k], cudaEventDisableTiming);

@@ -1,4 +1,4 @@
-// HostIo against a stand-in for the CUDA runtime, in which device
+// HostIo and PinPool against a stand-in for the CUDA runtime, in which device
 // memory cannot be touched by the host and a copy whose direction does not
 // match its pointers is refused.
 //   host_io copy BYTES KINDS   one call with two inputs and two outputs of BYTES
@@ -6,6 +6,7 @@
 //                              for each of the four.  Prints "ok" when every
 //                              output holds what the "kernel" wrote and it read
 //                              the inputs, or the CUDA error that refused the call
+//   host_io pool               blocks of the pool at its limits, and calls without
 #include "../../billardballraytracing3d_b200/csrc/host_io.hpp"
 
 #include <sys/mman.h>
@@ -15,6 +16,7 @@
 #include <cstdlib>
 #include <map>
 #include <string>
+#include <vector>
 
 namespace {
 
@@ -22,6 +24,7 @@ struct Mapping { size_t bytes; char* view; };   // device range, and a view of i
 std::map<char*, Mapping> device_memory;
 std::map<char*, size_t> pinned;
 std::mutex mu;
+int pin_calls = 0, pin_limit = 1 << 30;
 
 template <class M>
 auto find(M& m, const void* p, size_t (*size)(const typename M::mapped_type&)) {
@@ -64,6 +67,7 @@ cudaError_t cudaFree(void* p) {
 }
 cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) {
     std::lock_guard<std::mutex> g(mu);
+    if (++pin_calls > pin_limit) return cudaErrorMemoryAllocation;
     *p = std::malloc(bytes);
     pinned[static_cast<char*>(*p)] = bytes;
     return cudaSuccess;
@@ -146,5 +150,26 @@ int main(int argc, char** argv) {
         std::printf("%s\n", call(std::strtoull(argv[2], nullptr, 10), argv[3]).c_str());
         return 0;
     }
-    return 2;
+    // the pool at its limits
+    bbrt::PinPool& pool = bbrt::PinPool::get();
+    {
+        bbrt::PinPool::User user;
+        std::vector<char*> held[2];
+        for (int kind = 0; kind < 2; ++kind)
+            while (char* p = pool.take(kind)) held[kind].push_back(p);
+        std::printf("blocks %zu %zu pinned %zu\n", held[0].size(), held[1].size(), pinned.size());
+        // calls of every size class while all blocks are out: no more is pinned
+        const int before = pin_calls;
+        for (size_t bytes : { 1000, 100000, 3000000 }) std::printf("out %s\n", call(bytes, "hhhh").c_str());
+        std::printf("pinned by them %d\n", pin_calls - before);
+        for (int kind = 0; kind < 2; ++kind)
+            for (char* p : held[kind]) pool.give(kind, p);
+    }
+    std::printf("after the last scene %zu\n", pinned.size());
+    pin_limit = pin_calls;   // the system pins no more
+    {
+        bbrt::PinPool::User user;
+        for (size_t bytes : { 1000, 100000, 3000000 }) std::printf("none %s\n", call(bytes, "hhhh").c_str());
+    }
+    return 0;
 }

@@ -1,6 +1,6 @@
 """The staging of host arrays (csrc/host_io.hpp) against a stand-in for the CUDA
-runtime, on the CPU: every size class with pageable, pinned and device arrays in every
-place."""
+runtime, on the CPU: every size class with pageable, pinned and device arrays in
+every place, and the pinned pool at its limits."""
 import os
 import subprocess
 
@@ -38,3 +38,10 @@ def test_device_memory_is_left_to_the_cuda_copy(host_io, kinds):
     CUDA copy with the call's direction takes it or refuses it (here: refuses)."""
     for n in SIZES:
         assert host_io("copy", n, kinds)[0] == "error 1", n
+
+
+def test_pool_limits(host_io):
+    assert host_io("pool")[:-1] == ["blocks 16 4 pinned 20",
+                                    "out ok", "out ok", "out ok", "pinned by them 0",
+                                    "after the last scene 0",
+                                    "none ok", "none ok", "none ok"]
