@@ -446,6 +446,8 @@ int upload_node_tables(bbrt_scene* s, const std::vector<double>& nbox, const std
     return BBRT_OK;
 }
 
+bool node_tests_f32();   // the process-wide schedule's node_f32
+
 // The leaf tables of DScene (leaf records, and the leaf lists of ray_warp.cu)
 // of a scene or set whose object tables, leaf order and cull boxes are on the
 // device, from its breadth-first node arrays and the root of each tree; one
@@ -578,6 +580,7 @@ int build_leaf_tables(bbrt_scene* s, const std::vector<double>& nbox, const std:
     D.pair_node = reinterpret_cast<const int*>(d + at_pnode);
     D.m_ref = reinterpret_cast<const int*>(d + at_ref);
     D.leaf_lists = D.node_f32_ok && shallow ? 1 : 0;
+    D.node_f32 = node_tests_f32() ? 1 : 0;
     s->has_triangles = std::any_of(s->host.kind.begin(), s->host.kind.end(), [](int k) { return k != BBRT_OBJ_PATCH; });
     s->small_leaves = true;
     for (size_t l = 0; l < nl; ++l)
@@ -879,7 +882,8 @@ bbrt::MlpNet guess_net(bbrt_scene* s) {
 // round's runnable set.  Rounds end when no ray is waiting; a small last
 // set, and rays whose query needed more solves than the resolved list holds,
 // are finished by k_resume.
-// Finishes the rays of `reqs` (or `rays`) from their saved state.
+bool node_tests_f32() { return tuning().node_f32 != 0; }
+
 // The scene's schedule: its own once set or autotuned, else the library defaults.
 bbrt_tuning scene_tuning(const bbrt_scene* s) {
     if (s->tune_set) return s->tune;

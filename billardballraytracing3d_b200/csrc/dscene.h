@@ -49,6 +49,7 @@ struct DScene {
     // leaf_lists = 0: not usable (a box beyond the FP32 test's range, or a tree
     // so deep that a walk could overflow its stack).
     int leaf_lists = 0;
+    int node_f32 = 1;                      // 0: the warp-per-ray kernels test nodes in FP64 only
     const double* leaf_box = nullptr;
     const float4* leaf_node = nullptr;
     const int* leaf_rank = nullptr;

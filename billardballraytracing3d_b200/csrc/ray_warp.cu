@@ -343,7 +343,7 @@ __device__ __forceinline__ bool ray_query(const DScene& S, RayWork& w, const V3&
     const bool use_cull = cull_ok(S, member, cull_flag, o, d);
     const CullRay cr = make_cull_ray(S, member, o, d);
     NodeRay nr;
-    const bool node32 = make_node_ray(S, cr, nr);
+    const bool node32 = make_node_ray(S, cr, nr) && S.node_f32;
     // ---- leaves whose box the ray meets
     const int c_end = S.m_cut[member < 0 ? 1 : member + 1];
     int n_leaf = 0;
