@@ -104,6 +104,7 @@ struct bbrt_scene {
     bool device_ready = false;      // device, stream and events chosen
     bool has_triangles = false;
     bool small_leaves = false;      // no leaf has more slots than a split round takes
+    bool split_pays = false;        // split rounds are the faster ones (see split_pays())
     bool tables_uploaded = false;   // patch node / field tables on the device
     bool setup_on_device = false;   // coarse grids, cells and cull boxes computed on (and kept only on) the GPU
     int device = 0;
@@ -448,6 +449,16 @@ int upload_node_tables(bbrt_scene* s, const std::vector<double>& nbox, const std
 
 bool node_tests_f32();   // the process-wide schedule's node_f32
 
+bool mostly_triangles(const bbrt::HostScene& H) { return 1024LL * H.n_patches <= H.n_objects; }
+
+// Whether a scene's wavefronts are faster as split rounds than as k_advance
+// rounds: where its culling is in force (asked for, and the tables could be
+// made).  Without, no ray can be culled, and split rounds leave them all to the
+// warp-per-ray kernel: still the better way to stage 1 of every cell (131,072 rays
+// at spheres of radius 1,000: 3.3 ms against 3.7), but not for triangles (1,000 of
+// them, 131,072 and 1M rays: 0.67 and 4.9 ms against 0.23 and 0.96).
+bool split_pays(const bbrt_scene* s) { return s->cull.enabled || !mostly_triangles(s->host); }
+
 // The leaf tables of DScene (leaf records, and the leaf lists of ray_warp.cu)
 // of a scene or set whose object tables, leaf order and cull boxes are on the
 // device, from its breadth-first node arrays and the root of each tree; one
@@ -688,6 +699,7 @@ int ensure_uploaded(bbrt_scene* s) {
         if (reinterpret_cast<uintptr_t>(p) % 16 != 0)
             return fail(BBRT_ERR_CUDA, "bbrt_scene_upload: scene array not 16-byte aligned");
     if ((rc = build_leaf_tables(s, nbox, nlink, { 0 }))) return rc;
+    s->split_pays = split_pays(s);
     BBRT_CUDA(s->stats.ensure(sizeof(long long) * bbrt::ST_COUNT));
     BBRT_CUDA(s->work.ensure(sizeof(unsigned long long)));
     s->uploaded = true;
@@ -940,13 +952,23 @@ bool sort_round_requests(const bbrt_scene* s) {
 
 // Whether a wavefront runs split rounds (k_walk and k_stage1 of rounds.cu) or
 // k_advance rounds.  Split ones need the leaf lists, leaves of few slots and
-// culling; sample recording needs every patch of a visited leaf, in visiting
-// order; and the network knows no triangles.  Same box, split against
-// k_advance: see k_stage1.
+// culling, and have to be the faster ones (split_pays); sample recording needs
+// every patch of a visited leaf, in visiting order; and the network knows no
+// triangles.  Same box, split against k_advance: see k_stage1.
 bool split_rounds(const bbrt_scene* s, const bbrt::TraceArgs& A) {
     const bool learned = s->host.cfg.guess == BBRT_GUESS_LEARNED && s->guess.trained;
-    return s->dev.leaf_lists && s->small_leaves && s->host.cfg.cull && tuning().node_f32 && !A.samples &&
+    return s->dev.leaf_lists && s->small_leaves && s->host.cfg.cull && s->split_pays && tuning().node_f32 && !A.samples &&
            !(learned && s->has_triangles);
+}
+
+// Whether a batch of n BVH queries runs a thread per query (else a warp).  For a
+// scene of triangles from 24,576 queries on, where both take 0.13 ms (1,000
+// triangles; 65,536: 0.12 ms against 0.26; 1M: 0.87 against 2.9, with 100,000
+// triangles 1.8 against 6.1).  With a patch among a thousand triangles from
+// 65,536 on (4 patches and 100,000 triangles: 0.32 against 0.34, 1M: 2.2 against
+// 4.3; 192 patches, which the rays meet, 0.89 against 0.74 and 10.0 against 9.1).
+bool query_by_thread(const bbrt_scene* s, long long n) {
+    return mostly_triangles(s->host) && n >= (s->host.n_patches ? 65536 : 24576);
 }
 
 // Round 0's processing order (s->order): rays bucketed by where they enter
@@ -1757,12 +1779,16 @@ BBRT_API int bbrt_intersect(bbrt_scene_t s, const double* origins, const double*
     Q.mode = mode;
     Q.object = object;
     Q.cull = s->host.cfg.cull;
+    auto launch = [&]() -> int {
+        const bool warp = mode == BBRT_QUERY_BVH && !query_by_thread(s, n);
+        BBRT_CUDA(warp ? bbrt::launch_query_warp(s->dev, Q, s->sm_count, st) : bbrt::launch_query(s->dev, Q, st));
+        return BBRT_OK;
+    };
     if (flags & BBRT_DEVICE_PTRS) {
         Q.origins = origins;
         Q.dirs = dirs;
         Q.out = out;
-        BBRT_CUDA((mode == BBRT_QUERY_BVH ? bbrt::launch_query_warp(s->dev, Q, s->sm_count, st) : bbrt::launch_query(s->dev, Q, st)));
-        return BBRT_OK;
+        return launch();
     }
     const size_t vb = sizeof(double) * 3 * static_cast<size_t>(n);
     bbrt::HostIo io(s->io, s->slot_ev, s->device, st);
@@ -1777,7 +1803,7 @@ BBRT_API int bbrt_intersect(bbrt_scene_t s, const double* origins, const double*
     if (mode == BBRT_QUERY_BVH && n >= wave_min(s) && split_rounds(s, bbrt::TraceArgs())) {
         if ((rc = run_query_rounds(s, Q.origins, Q.dirs, n, io.at<bbrt_hit>(h), st))) return rc;
     } else {
-        BBRT_CUDA(mode == BBRT_QUERY_BVH ? bbrt::launch_query_warp(s->dev, Q, s->sm_count, st) : bbrt::launch_query(s->dev, Q, st));
+        if ((rc = launch())) return rc;
     }
     BBRT_CUDA(io.close());
     return BBRT_OK;
@@ -3091,6 +3117,7 @@ int build_scene_set(const std::vector<bbrt_scene*>& mem, bbrt_scene_set* set) {
     }
     BBRT_CUDA(cudaStreamSynchronize(S.stream));
     if ((rc = build_leaf_tables(&S, nbox, nlink, roots))) return rc;
+    S.split_pays = std::all_of(mem.begin(), mem.end(), [](const bbrt_scene* m) { return m->split_pays; });
     BBRT_CUDA(S.stats.ensure(sizeof(long long) * bbrt::ST_COUNT));
     BBRT_CUDA(S.work.ensure(sizeof(unsigned long long)));
     S.tables_uploaded = true;

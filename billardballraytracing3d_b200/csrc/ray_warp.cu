@@ -456,10 +456,14 @@ __device__ __forceinline__ bool ray_query(const DScene& S, RayWork& w, const V3&
             w.leaf_pos[at] = pos;
         }
         __syncwarp();
-        const Stage1 mine = ray_stage1(S, w, P, o, d, use_cull, cr, lane, ctr);
-        // ---- stage-1 hits (and triangles) in order
-        for (unsigned hits = __ballot_sync(kFull, lane < P && (mine.have || w.sub[lane < P ? lane : 0] < 0)); hits;
-             hits &= hits - 1) {
+        Stage1 mine = ray_stage1(S, w, P, o, d, use_cull, cr, lane, ctr);
+        if (lane < P && w.sub[lane] < 0) {   // triangles: a lane each
+            double u, v;
+            const double* tv = S.tri + static_cast<long long>(~w.sub[lane]) * 9;
+            mine.have = mt_full(o, d, load3(tv), load3(tv + 3), load3(tv + 6), mine.t, u, v);
+        }
+        // ---- hits in order
+        for (unsigned hits = __ballot_sync(kFull, lane < P && mine.have); hits; hits &= hits - 1) {
             const int c = __ffs(hits) - 1;
             const int lp = w.leaf_pos[c];
             if (lp != open) {
@@ -469,6 +473,7 @@ __device__ __forceinline__ bool ray_query(const DScene& S, RayWork& w, const V3&
             const int sub = w.sub[c];
             const double t0 = __shfl_sync(kFull, mine.t, c);
             const int key = __shfl_sync(kFull, mine.key, c);
+            if (sub < 0 && !(t0 < best_t)) continue;
             QHit h;
             h.err = 0;
             h.ev0 = h.ev1 = 0.0;

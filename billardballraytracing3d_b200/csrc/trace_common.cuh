@@ -356,7 +356,9 @@ __device__ __forceinline__ int object_intersect(const DScene& S, int obj, const 
 // BVH::intersect with a 64-entry stack.  Returns the closest hit (obj >= 0),
 // a miss (obj < 0, err 0), or the first Newton failure met (err != 0).
 // off_patch_miss (learned form): a Newton root outside its patch is a miss.
-template <class Ctr>
+// PATCHES false: a scene of triangles only (without stage 1 and the Newton solve
+// a query kernel needs 96 registers and spills none).
+template <bool PATCHES = true, class Ctr>
 __device__ QHit bvh_query(const DScene& S, const V3& o, const V3& d, int cull_flag, Ctr& ctr,
                           bool off_patch_miss = false, int member = -1) {
     QHit best;
@@ -382,13 +384,15 @@ __device__ QHit bvh_query(const DScene& S, const V3& o, const V3& d, int cull_fl
             for (int k = 0; k < count; ++k) {
                 const LeafRec rec = load_leaf(S, start + k);
                 const int obj = rec.obj();
-                if (use_cull && rec.sub() >= 0 && !cull_leaf(rec, cr)) {
+                if (PATCHES && use_cull && rec.sub() >= 0 && !cull_leaf(rec, cr)) {
                     ++ctr.patch_tests;
                     ++ctr.cell_tests;
                     continue;
                 }
                 QHit h;
-                const int r = object_intersect(S, obj, o, d, use_cull, cr, h, ctr);
+                int r;
+                if constexpr (PATCHES) r = object_intersect(S, obj, o, d, use_cull, cr, h, ctr);
+                else r = triangle_intersect(S, ~rec.sub(), o, d, h, ctr);
                 if (off_patch_miss && h.err == BBRT_RAY_NEWTON_DOMAIN) {
                     ++ctr.off_patch;
                     continue;

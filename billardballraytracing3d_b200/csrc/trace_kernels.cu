@@ -233,6 +233,16 @@ __global__ void __launch_bounds__(128) k_resume(DScene S, TraceArgs A, WaveArgs 
     flush_stats(A, ctr, tally, true);
 }
 
+// One BVH query per thread.
+template <bool PATCHES>
+__global__ void __launch_bounds__(128) k_query_bvh(DScene S, QueryArgs Q) {
+    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (i >= Q.n) return;
+    CountersT<false> ctr;
+    write_hit(static_cast<bbrt_hit*>(Q.out) + i,
+              bvh_query<PATCHES>(S, load3(Q.origins + 3 * i), load3(Q.dirs + 3 * i), Q.cull, ctr));
+}
+
 // One query per thread: brute force over all objects, or one object.
 __global__ void __launch_bounds__(128) k_query(DScene S, QueryArgs Q) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -619,8 +629,10 @@ cudaError_t launch_node_check(const DScene& S, const double* o, const double* d,
 
 cudaError_t launch_query(const DScene& S, const QueryArgs& Q, cudaStream_t stream) {
     if (Q.n <= 0) return cudaSuccess;
-    const long long blocks = (Q.n + 127) / 128;
-    k_query<<<static_cast<unsigned>(blocks), 128, 0, stream>>>(S, Q);
+    const unsigned blocks = static_cast<unsigned>((Q.n + 127) / 128);
+    if (Q.mode != BBRT_QUERY_BVH) k_query<<<blocks, 128, 0, stream>>>(S, Q);
+    else if (S.max_nodes > 0) k_query_bvh<true><<<blocks, 128, 0, stream>>>(S, Q);
+    else k_query_bvh<false><<<blocks, 128, 0, stream>>>(S, Q);
     return cudaGetLastError();
 }
 
