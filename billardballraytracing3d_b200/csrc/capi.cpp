@@ -1509,6 +1509,19 @@ int run_trace_device(bbrt_scene* s, const double* d_o, const double* d_d, long l
     return rc;
 }
 
+// The most queries run as one set of rounds: their workspace, 0.6 KB a query, is
+// several times the rays and records of the call, so it does not grow with the
+// batch (4M queries: 2.6 GB).
+constexpr long long kQueryRounds = 4LL << 20;
+
+// The rounds' workspace for n queries, if the device has the memory.
+bool query_rounds_fit(bbrt_scene* s, long long n) {
+    const bool ok = s->wave.ensure(bbrt::split_workspace_bytes(n)) == cudaSuccess &&
+                    s->order_ws.ensure(bbrt::ray_order_workspace_bytes(n)) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
 // BVH queries as split rounds (always FP64 from the stage-1 triangle, whatever
 // the scene's modes); waits for them.
 int run_query_rounds(bbrt_scene* s, const double* d_o, const double* d_d, long long n, bbrt_hit* out, cudaStream_t st) {
@@ -1800,8 +1813,12 @@ BBRT_API int bbrt_intersect(bbrt_scene_t s, const double* origins, const double*
     Q.out = io.at<bbrt_hit>(h);
     // many queries: as rounds, like a trace of as many rays (200,003 tetrahedron
     // queries: 1.87 ms a warp per query, about 0.55 ms as rounds)
-    if (mode == BBRT_QUERY_BVH && n >= wave_min(s) && split_rounds(s, bbrt::TraceArgs())) {
-        if ((rc = run_query_rounds(s, Q.origins, Q.dirs, n, io.at<bbrt_hit>(h), st))) return rc;
+    if (mode == BBRT_QUERY_BVH && n >= wave_min(s) && split_rounds(s, bbrt::TraceArgs()) &&
+        query_rounds_fit(s, std::min(n, kQueryRounds))) {
+        for (long long at = 0; at < n; at += kQueryRounds)
+            if ((rc = run_query_rounds(s, Q.origins + 3 * at, Q.dirs + 3 * at, std::min(kQueryRounds, n - at),
+                                       io.at<bbrt_hit>(h) + at, st)))
+                return rc;
     } else {
         if ((rc = launch())) return rc;
     }

@@ -40,3 +40,35 @@ def test_schedules_do_not_change_query_results(nested, graph_rounds, warp_tail, 
     got = sc.intersect(o, d)
     for k in KEYS:
         assert np.array_equal(got[k], ref[k], equal_nan=True), k
+
+
+def test_workspace_does_not_grow_with_the_batch(built):
+    """9M queries at two spheres: device memory taken by the call beyond its rays
+    and records (152 bytes a query), and records equal to a warp per query's."""
+    import ctypes
+    import torch
+    n = 9000001
+    sc = api.Scene(scenes.scene_two_spheres(), config=C.default_config(coarse_grid_n=9, newton_tol=1e-12))
+    rng = np.random.Generator(np.random.PCG64(5))
+    o = rng.uniform(-3.0, 3.0, (n, 3))
+    o[:, 2] = 4.0
+    d = np.zeros((n, 3))
+    d[:, :2] = rng.uniform(-0.3, 0.3, (n, 2))
+    d[:, 2] = -0.9
+    torch.cuda.init()
+    sc.intersect(o[:64], d[:64])
+    free = torch.cuda.mem_get_info()[0]
+    got = sc.intersect(o, d)
+    taken = free - torch.cuda.mem_get_info()[0]
+    assert taken - 152 * n < 3.5e9, taken
+    to, td = torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda()
+    hits = torch.zeros(n * C.HIT_DTYPE.itemsize, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    C.check(sc.lib, sc.lib.bbrt_intersect(sc.h, ctypes.c_void_p(to.data_ptr()), ctypes.c_void_p(td.data_ptr()), n,
+                                          C.QUERY_BVH, 0, C.DEVICE_PTRS, ctypes.c_void_p(hits.data_ptr()), None),
+            "bbrt_intersect")
+    torch.cuda.synchronize()
+    ref = hits.cpu().numpy().view(C.HIT_DTYPE)
+    assert (ref["object"] >= 0).sum() > n // 10
+    for k in KEYS:
+        assert np.array_equal(got[k], ref[k], equal_nan=True), k
