@@ -1523,11 +1523,14 @@ bool query_rounds_fit(bbrt_scene* s, long long n) {
 }
 
 // BVH queries as split rounds (always FP64 from the stage-1 triangle, whatever
-// the scene's modes); waits for them.
+// the scene's modes, and with the default watchdog: a schedule's bounds its
+// traces); waits for them.
 int run_query_rounds(bbrt_scene* s, const double* d_o, const double* d_d, long long n, bbrt_hit* out, cudaStream_t st) {
     const int precision = s->dev.precision, guess = s->host.cfg.guess;
+    const long long watchdog = s->tune.watchdog_cycles;
     s->dev.precision = BBRT_PREC_FP64;
     s->host.cfg.guess = BBRT_GUESS_TRIANGLE;
+    s->tune.watchdog_cycles = 0;
     bbrt::TraceArgs A;
     int rc = prepare_trace(s, d_o, d_d, n, 1, nullptr, nullptr, 1, st, false, A);
     A.query_out = out;
@@ -1540,6 +1543,7 @@ int run_query_rounds(bbrt_scene* s, const double* d_o, const double* d_d, long l
     }
     s->dev.precision = precision;
     s->host.cfg.guess = guess;
+    s->tune.watchdog_cycles = watchdog;
     return rc;
 }
 

@@ -72,3 +72,16 @@ def test_workspace_does_not_grow_with_the_batch(built):
     assert (ref["object"] >= 0).sum() > n // 10
     for k in KEYS:
         assert np.array_equal(got[k], ref[k], equal_nan=True), k
+
+
+@pytest.mark.parametrize("graph_rounds", [1, 0])
+def test_a_watchdog_set_for_traces_does_not_stop_queries(nested, graph_rounds):
+    patches, cfg, o, d, ref = nested
+    sc = api.Scene(patches, config=cfg)
+    sc.tuning(graph_rounds=graph_rounds, wave_min_rays=1, watchdog_cycles=1)
+    got = sc.intersect(o, d)
+    for k in KEYS:
+        assert np.array_equal(got[k], ref[k], equal_nan=True), k
+    assert sc.tuning()["watchdog_cycles"] == 1
+    with pytest.raises(RuntimeError, match="watchdog"):
+        sc.trace(o, d, 30)
