@@ -928,6 +928,10 @@ long long wave_min(const bbrt_scene* s) {
     return plain && !tuning().wave_min_set ? 32768 : tuning().wave_min_rays;
 }
 
+// Whether the scene's rounds choose themselves if rays are ordered: no schedule
+// was set, autotuned or given by the environment.
+bool orders_by_itself(const bbrt_scene* s) { return !s->tune_set && !tuning().order_set; }
+
 // Whether a trace of n rays on device arrays has finished when its call
 // returns: from the schedule's wavefront size on, whichever kernels run it.
 bool waits_for_trace(const bbrt_scene* s, long long n) { return n >= scene_tuning(s).wave_min_rays; }
@@ -1249,7 +1253,7 @@ struct WaveRun {
         // them more than coherent walks give (4M-ray ellipsoid trace: first walk
         // 1.04 ms as they come, 1.50 ms and 0.25 ms of sorting ordered; 1M-ray
         // tetrahedron trace 0.23 against 0.29 and 0.05 ms).
-        if (split && !s->tune_set && !tuning().order_set) T.order_rays = 0;
+        if (split && orders_by_itself(s)) T.order_rays = 0;
         BBRT_CUDA(s->wave.ensure(split ? bbrt::split_workspace_bytes(n) : bbrt::wave_workspace_bytes(n)));
         BBRT_CUDA(s->wave_ctr.ensure(bbrt::kWaveCounters * sizeof(unsigned int)));
         if (!s->wave_ctr_host)
@@ -2727,13 +2731,16 @@ BBRT_API int bbrt_scene_autotune(bbrt_scene_t s, const double* origins, const do
         ms = total / trials;
         return BBRT_OK;
     };
+    // coordinate descent from the schedule in force: launch shape (of k_advance,
+    // where it runs the rounds), then tail size
+    const bool split = split_rounds(s, bbrt::TraceArgs());
     bbrt_tuning cur = scene_tuning(s);
+    if (split && orders_by_itself(s)) cur.order_rays = 0;
     double cur_ms = 0.0;
     rc = time_one(cur, cur_ms);
-    // coordinate descent: launch shape, then tail size
     const int shapes[] = { 3, 6, 1, 0 };
     for (int sh : shapes) {
-        if (rc || sh == cur.advance_shape) continue;
+        if (rc || split || sh == cur.advance_shape) continue;
         bbrt_tuning c = cur;
         c.advance_shape = sh;
         double ms = 0.0;

@@ -458,7 +458,7 @@ BBRT_API int bbrt_scene_get_tuning(bbrt_scene_t scene, bbrt_tuning* out);
 BBRT_API int bbrt_scene_set_tuning(bbrt_scene_t scene, const bbrt_tuning* tuning);
 /* Times candidate schedules on the given rays (host arrays; the scene's
  * current precision and guess modes), by coordinate descent over the launch
- * shape, then the tail size, then ordered or unordered rays, then graph-launched vs
+ * shape (where k_advance runs the rounds), then the tail size, then ordered or unordered rays, then graph-launched vs
  * host-driven rounds, `trials` timed traces each after one untimed
  * one; keeps the fastest in the scene and returns it with its mean device
  * time per trace. */
