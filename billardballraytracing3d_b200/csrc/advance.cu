@@ -217,64 +217,38 @@ __device__ __forceinline__ void batch_stage1(const DScene& S, WarpWork& w, unsig
     __syncwarp();
     const int hi = hl / NB, hj = hl - hi * NB;
     int n_blk = 0;
-    // four patches per half-warp with their boxes loaded together: the loads'
-    // latency, not the tests, is what a batch waits for
-    constexpr int U = 1;
-    for (int p = 0; p < P; p += 2 * U) {
-        int owner[U];
-        float2 b[U][3];
-#pragma unroll
-        for (int k = 0; k < U; ++k) {
-            const int c = p + 2 * k + half;
-            owner[k] = c < P && hl < NB2 ? w.lane_of[c] : -1;
-            if (owner[k] >= 0) {
-                const int pidx = __float_as_int(w.cr_b[owner[k]].w);
-                const float2* src = reinterpret_cast<const float2*>(S.c_block_box + (static_cast<long long>(pidx) * NB2 + hl) * 6);
-#pragma unroll
-                for (int a = 0; a < 3; ++a) b[k][a] = src[a];
-            }
+    for (int p = 0; p < P; p += 2) {
+        const int c = p + half;
+        const int owner = c < P && hl < NB2 ? w.lane_of[c] : -1;
+        bool pass = false;
+        if (owner >= 0) {
+            const int pidx = __float_as_int(w.cr_b[owner].w);
+            pass = cull_box(S.c_block_box + (static_cast<long long>(pidx) * NB2 + hl) * 6, work_cull_ray(w, owner));
         }
-#pragma unroll
-        for (int k = 0; k < U; ++k) {
-            const bool pass = owner[k] >= 0 && cull_box(b[k][0], b[k][1], b[k][2], work_cull_ray(w, owner[k]));
-            const unsigned m = __ballot_sync(kFull, pass);
-            if (pass) w.blk[n_blk + __popc(m & lt)] = static_cast<unsigned short>(owner[k] << 8 | hi << 4 | hj);
-            n_blk += __popc(m);
-        }
+        const unsigned m = __ballot_sync(kFull, pass);
+        if (pass) w.blk[n_blk + __popc(m & lt)] = static_cast<unsigned short>(owner << 8 | hi << 4 | hj);
+        n_blk += __popc(m);
     }
     __syncwarp();
     int n_cell = 0;
-    constexpr int V = 1;
-    for (int p = 0; p < n_blk; p += 2 * V) {
-        int entry[V];   // owner << 8 | row << 4 | column, or -1
-        float2 b[V][3];
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-            const int c = p + 2 * k + half;
-            entry[k] = -1;
-            if (c < n_blk) {
-                const int e = w.blk[c], i = ((e >> 4) & 15) * 4 + (hl >> 2), j = (e & 15) * 4 + (hl & 3);
-                if (i < nc && j < nc) {
-                    entry[k] = (e & ~255) | i << 4 | j;
-                    const int pidx = __float_as_int(w.cr_b[e >> 8].w);
-                    const float2* src = reinterpret_cast<const float2*>(S.c_cell_box +
-                                                                        (static_cast<long long>(pidx) * nc * nc + i * nc + j) * 6);
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) b[k][a] = src[a];
-                }
+    for (int p = 0; p < n_blk; p += 2) {
+        const int c = p + half;
+        int entry = 0;   // owner << 8 | row << 4 | column
+        bool pass = false;
+        if (c < n_blk) {
+            const int e = w.blk[c], owner = e >> 8, i = ((e >> 4) & 15) * 4 + (hl >> 2), j = (e & 15) * 4 + (hl & 3);
+            if (i < nc && j < nc) {
+                entry = (e & ~255) | i << 4 | j;
+                if (STATS) atomicAdd(&w.cells[owner], 1);
+                const int pidx = __float_as_int(w.cr_b[owner].w);
+                pass = cull_box(S.c_cell_box + (static_cast<long long>(pidx) * nc * nc + i * nc + j) * 6, work_cull_ray(w, owner));
+                if (STATS && pass) atomicAdd(&w.tris[owner], 6);
             }
         }
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-            const int owner = entry[k] >> 8;
-            if (STATS && entry[k] >= 0) atomicAdd(&w.cells[owner], 1);
-            const bool pass = entry[k] >= 0 && cull_box(b[k][0], b[k][1], b[k][2], work_cull_ray(w, owner));
-            if (STATS && pass) atomicAdd(&w.tris[owner], 6);
-            const unsigned m = __ballot_sync(kFull, pass);
-            if (pass) w.cell[n_cell + __popc(m & lt)] = static_cast<unsigned short>(entry[k]);
-            n_cell += __popc(m);
-        }
-        if (n_cell > kCellFlush && p + 2 * V < n_blk) {
+        const unsigned m = __ballot_sync(kFull, pass);
+        if (pass) w.cell[n_cell + __popc(m & lt)] = static_cast<unsigned short>(entry);
+        n_cell += __popc(m);
+        if (n_cell > kCellFlush && p + 2 < n_blk) {
             __syncwarp();
             batch_tris<STATS>(S, w, n_cell, lane, mine);
             __syncwarp();

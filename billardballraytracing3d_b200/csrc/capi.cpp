@@ -115,8 +115,7 @@ struct bbrt_scene {
     bool in_flight = false;         // ... where there was one
     std::vector<void*> allocs;
     long long device_bytes = 0;
-    DevBuf stats, work, in_o, in_d, o_status, o_bounce, o_dir, o_end, o_hobj, o_hpt, o_huv, o_eobj, o_eval,
-        counts, hits, wave, wave_ctr, o_work, order, order_ws, io;
+    DevBuf stats, work, in_o, in_d, o_status, o_bounce, counts, hits, wave, wave_ctr, order, order_ws, io;
     cudaEvent_t slot_ev[bbrt::PinPool::kSlots] = {};   // one per copying thread of HostIo
     bbrt::PinPool::User pin_user;
     unsigned int* wave_ctr_host = nullptr;   // pinned copy of the round counters
@@ -167,8 +166,7 @@ struct bbrt_scene {
 
     ~bbrt_scene() {
         for (void* p : allocs) cudaFree(p);
-        for (DevBuf* b : { &stats, &work, &in_o, &in_d, &o_status, &o_bounce, &o_dir, &o_end, &o_hobj, &o_hpt,
-                           &o_huv, &o_eobj, &o_eval, &counts, &hits, &wave, &wave_ctr, &o_work, &order, &order_ws, &io,
+        for (DevBuf* b : { &stats, &work, &in_o, &in_d, &o_status, &o_bounce, &counts, &hits, &wave, &wave_ctr, &order, &order_ws, &io,
                            &guess.P, &guess.G, &guess.m1, &guess.m2, &guess.image, &guess.loss, &guess.err,
                            &guess.out, &guess.rows })
             b->release();
@@ -825,8 +823,8 @@ cudaError_t timed(bbrt_scene* s, int kind, cudaStream_t st, F&& launch) {
 }
 
 // Batches at least this large run as a wavefront of advance / Newton rounds;
-// smaller ones (and the last few rays of a wavefront) run one ray per thread
-// to the end.
+// smaller ones (and the last few rays of a wavefront) run one ray per warp to
+// the end.
 struct Tuning {
     long long wave_min_rays = 8192;   // smaller batches: one ray per warp to the end (see wave_min)
     bool wave_min_set = false;        // ... given by the environment

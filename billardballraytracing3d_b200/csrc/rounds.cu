@@ -282,9 +282,12 @@ constexpr int kBlkCap = 128, kCellCap = 64;   // larger grids: blocks and cells 
 // (delta - o) i for the max face.  Rounding: o, o + delta and the product in p
 // 3 units of 2^-24 (|o| + delta) |i|, 1/d 2 of (|b| + |o| + delta) |i|, the sum
 // 1: 6 (|b| + |o| + delta), as a distance, of the 32 that delta holds for the
-// slab test (cull_constants).  |i| is kept to 1e18, so that an axis the ray does
-// not move along decides by where the origin is; a time of at most t moves it
-// t * 1e-18 there.
+// slab test (cull_constants).  |i| is kept to 1e18, which is sound on the axes
+// that it cuts off (|d_a| < 1e-18): a triangle is hit only with |det| >= 1e-9, so
+// |d| >= 1e-9 / h^2 (h: cull_h, at least the longest edge) and the hit's
+// t <= 1e9 h^2 L; up to it the ray moves less than 1e-9 h^2 L on such an axis, and
+// delta holds cull_a L = 2.8e-5 h^2 L, so the origin is that far inside the
+// inflated slab and the times cut off still contain [0, t].
 struct __align__(16) CullFma {
     float ix, iy, iz, nx, ny, nz, xx, xy, xz, pad[3];
 };
@@ -367,8 +370,8 @@ __device__ __forceinline__ void s1_tris(const DScene& S, S1Work& w, int n_cells,
 }
 
 // Stage 1 of candidates [first, last) by their patches' quadtrees: every step
-// takes eight waiting nodes of one level and tests their four children, a lane
-// each, or sixteen cells' triangles; the deepest level with enough waiting goes
+// takes sixteen waiting nodes of one level and tests their four children, two a
+// lane, or sixteen cells' triangles; the deepest level with enough waiting goes
 // first, so the lists stay short and the lanes full (5.3 tests a level and
 // candidate where sixteen blocks and sixteen cells a block were 32).
 template <bool STATS>

@@ -551,7 +551,7 @@ BBRT_API int bbrt_node_test_check(const double* o, const double* d, const double
  * owns every input and output (device arrays), and the scene must already be
  * on the device (bbrt_scene_upload, or any earlier compute call).
  *
- * It traces like bbrt_trace with BBRT_DEVICE_PTRS, always one GPU thread per
+ * It traces like bbrt_trace with BBRT_DEVICE_PTRS, always one warp per
  * ray to the end.  Its scratch — the ray counter, the statistics block and,
  * when hit_counts is not NULL, one hit counter per object — lives in a
  * static device array of the library, one per device, held until the process
