@@ -3136,7 +3136,7 @@ int build_scene_set(const std::vector<bbrt_scene*>& mem, bbrt_scene_set* set) {
     if ((rc = join_device(S, pf32, D.p_fields32))) return rc;
     if ((rc = join_device(S, cx, D.c_xyz))) return rc;
     if ((rc = join_device(S, cc, D.c_cell))) return rc;
-    if ((rc = join_device(S, tr, D.tri))) return rc;
+    if (tri_off[M] > 0 && (rc = join_device(S, tr, D.tri))) return rc;   // (null: no triangles)
     if (cull_blocks) {
         if ((rc = join_device(S, cb, D.c_cell_box))) return rc;
         if ((rc = join_device(S, bb, D.c_block_box))) return rc;
