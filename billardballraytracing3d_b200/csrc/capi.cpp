@@ -111,8 +111,8 @@ struct bbrt_scene {
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[4] = { nullptr, nullptr, nullptr, nullptr };
-    cudaEvent_t busy = nullptr;     // the end of the last trace that returned with its work in flight ...
-    bool in_flight = false;         // ... where there was one
+    bool in_flight = false;         // a trace has returned with its work in flight, up to ev[1]
+    bool capturing = false;         // the call's stream is under capture
     std::vector<void*> allocs;
     long long device_bytes = 0;
     DevBuf stats, work, in_o, in_d, o_status, o_bounce, counts, hits, wave, wave_ctr, order, order_ws, io;
@@ -171,7 +171,6 @@ struct bbrt_scene {
                            &guess.out, &guess.rows })
             b->release();
         if (wave_ctr_host) cudaFreeHost(wave_ctr_host);
-        if (busy) cudaEventDestroy(busy);
         for (auto& e : slot_ev)
             if (e) cudaEventDestroy(e);
         for (WaveGraph& g : wgraphs) {
@@ -294,7 +293,6 @@ int ensure_device(bbrt_scene* s) {
     BBRT_CUDA(bbrt::noalloc_prepare());
     for (auto& e : s->ev) BBRT_CUDA(cudaEventCreate(&e));
     for (auto& e : s->kev) BBRT_CUDA(cudaEventCreate(&e));
-    BBRT_CUDA(cudaEventCreateWithFlags(&s->busy, cudaEventDisableTiming));
     s->device_ready = true;
     return BBRT_OK;
 }
@@ -1400,23 +1398,15 @@ int check_guess_waits(bbrt_scene* s, cudaStream_t st) {
 
 // Orders `st` after the scene's last trace, whose work may still run on another
 // stream: all traces of a scene hand out rays through one counter and count in
-// one statistics block, which each call clears.  A stream under capture cannot
-// wait for work outside it: ordering its replays is the caller's.
+// one statistics block, which each call clears.  Every trace ends with ev[1], so
+// one wait covers those before it too.  A stream under capture cannot wait for
+// work outside it, and its events mean nothing outside: such a call records none,
+// and ordering its replays is the caller's.
 int after_last_trace(bbrt_scene* s, cudaStream_t st) {
-    if (!s->in_flight) return BBRT_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     BBRT_CUDA(cudaStreamIsCapturing(st, &cap));
-    if (cap == cudaStreamCaptureStatusNone) BBRT_CUDA(cudaStreamWaitEvent(st, s->busy, 0));
-    return BBRT_OK;
-}
-
-// The call returns with its trace in flight on `st` (see after_last_trace).
-int leave_in_flight(bbrt_scene* s, cudaStream_t st) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    BBRT_CUDA(cudaStreamIsCapturing(st, &cap));
-    if (cap != cudaStreamCaptureStatusNone) return BBRT_OK;
-    BBRT_CUDA(cudaEventRecord(s->busy, st));
-    s->in_flight = true;
+    s->capturing = cap != cudaStreamCaptureStatusNone;
+    if (s->in_flight && !s->capturing) BBRT_CUDA(cudaStreamWaitEvent(st, s->ev[1], 0));
     return BBRT_OK;
 }
 
@@ -1467,13 +1457,13 @@ int prepare_trace(bbrt_scene* s, const double* d_o, const double* d_d, long long
     s->kspans.clear();
     s->rounds = 0;
     s->launches = 0;
-    BBRT_CUDA(cudaEventRecord(s->ev[0], st));
+    if (!s->capturing) BBRT_CUDA(cudaEventRecord(s->ev[0], st));
     return BBRT_OK;
 }
 
 // Records the call's end event and queues the statistics readback.
 int complete_trace(bbrt_scene* s, cudaStream_t st, bool want_stats, long long* host_stats, float* kernel_ms) {
-    BBRT_CUDA(cudaEventRecord(s->ev[1], st));
+    if (!s->capturing) BBRT_CUDA(cudaEventRecord(s->ev[1], st));
     if (want_stats) {
         BBRT_CUDA(cudaMemcpyAsync(host_stats, s->stats.p, sizeof(long long) * bbrt::ST_COUNT,
                                   cudaMemcpyDeviceToHost, st));
@@ -1493,6 +1483,8 @@ int run_trace_device(bbrt_scene* s, const double* d_o, const double* d_d, long l
     bbrt::TraceArgs A;
     int rc = prepare_trace(s, d_o, d_d, n, max_bounces, out_dev, hit_counts, count_from, st, want_stats, A);
     if (rc) return rc;
+    if (s->capturing && (waits_for_trace(s, n) || want_stats || kernel_ms))
+        return fail(BBRT_ERR_CUDA, "bbrt_trace: a call that waits for its trace cannot run on a stream under capture");
     GraphLaunch graph;
     if (n < wave_min(s)) {
         BBRT_CUDA(timed(s, K_TAIL, st, [&] { return bbrt::launch_rays(s->dev, A, bbrt::WaveArgs(), nullptr, nullptr, n, s->sm_count, st); }));
@@ -1856,7 +1848,7 @@ BBRT_API int bbrt_trace(bbrt_scene_t s, const double* origins, const double* dir
                               stats ? &kms : nullptr);
         s->time_kernels = false;
         if (rc) return rc;
-        if (!waits_for_trace(s, n) && (rc = leave_in_flight(s, st))) return rc;
+        if (!waits_for_trace(s, n) && !s->capturing) s->in_flight = true;
         if (stats) {
             BBRT_CUDA(cudaStreamSynchronize(st));
             fill_stats(s, hs, n, kms, kms, stats);

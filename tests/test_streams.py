@@ -74,7 +74,7 @@ def test_device_call_of_wavefront_size_has_finished_when_it_returns(tetra, n):
 def test_captured_call_replays_beside_other_calls(tetra):
     """A small device call captured on a stream: the capture neither waits for
     the call in flight before it nor leaves anything behind that a call outside
-    could wait for."""
+    could wait for.  A call that waits for its trace is refused in a capture."""
     import torch
     sc, work = tetra
     _, _, to, td, ref = work[0]
@@ -87,6 +87,9 @@ def test_captured_call_replays_beside_other_calls(tetra):
     torch.cuda.synchronize()
     call(pre, st.cuda_stream)
     with torch.cuda.graph(g, stream=st):
+        with pytest.raises(RuntimeError, match="capture"):
+            sc.trace_device(work[1][2].data_ptr(), work[1][3].data_ptr(), N[1], 200, {},
+                            stream=torch.cuda.current_stream().cuda_stream)
         call(cap, torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     g.replay()
