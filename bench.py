@@ -218,7 +218,8 @@ def advance_roofline(st, fp64_peak, fp32_peak, l2_peak):
             "note": "algorithmic work of the advance kernels (k_walk and k_stage1) of one step (device counters) over "
                     "their summed CUDA-event time; peaks: FP64/FP32 FMA and L2-resident reads measured in this process "
                     f"(bbrt_measure_pipe_peak), of measured; HBM {HBM_PEAK_GBS:.0f} GB/s, of {HBM_PEAK_SOURCE} "
-                    f"({'MEASURED_PEAKS.json' if HBM_PEAK_SOURCE == 'measured' else 'no MEASURED_PEAKS.json: the pool fallback'}); the exact FP64 "
+                    f"({'MEASURED_PEAKS.json' if HBM_PEAK_SOURCE == 'measured' else 'no MEASURED_PEAKS.json: the pool fallback'}), "
+                    "of algorithmic bytes, most of which L1 and L2 serve (DRAM bytes: traffic); the exact FP64 "
                     "path runs unfused mul/add (half the FMA peak at most); traffic per round from the ncu "
                     "capture in profiles/, scaled by node tests"}
 
